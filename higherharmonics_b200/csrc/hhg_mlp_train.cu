@@ -12,9 +12,12 @@
 //
 //   forward     Z_l = H_{l-1} W_l^T + b_l,  H_l = SiLU(Z_l)        (M = rows, N = 64)
 //   output      y = H_3 w_4 + b_4, loss = mean (y - T)^2           (CUDA cores, 64 -> 1)
-//   data grad   dH_{l-1} = dZ_l W_l,  dZ_{l-1} = dH_{l-1} SiLU'(Z_{l-1})  (N = 64 or 16)
-//   weight grad dW_l = dZ_l^T H_{l-1} over a 64-row chunk, M padded to 128
+//   data grad   dH_{l-1} = dZ_l W_l,  dZ_{l-1} = dH_{l-1} SiLU'(Z_{l-1})  (N = 64)
+//   weight grad dW_l = dZ_l^T H_{l-1} over the tile's 128 rows, M padded to 128
 //   Adam on FP32 master weights, then BF16 copies [n][k] and [k][n].
+//
+// One kernel carries a tile through all of it (mlp_step_kernel); the
+// optimiser is the only other launch of a step.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -34,7 +37,6 @@ constexpr int kH = hhg::kMlpH;          // 64
 constexpr int kIn = hhg::kMlpIn;        // 8
 constexpr int kInPad = hhg::kMlpInPad;  // 16
 constexpr int kRows = 128;              // rows per tile (M)
-constexpr int kChunk = 64;              // batch rows per weight-gradient tile (K)
 constexpr long long kSpin = 1ll << 24;  // bounded mbarrier polls
 
 // FP32 master parameters on the device (the first layer's inputs padded to 16)
@@ -122,22 +124,27 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, int ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" : : "r"(taddr), "r"(ncols) : "memory");
 }
 
-// 32 lanes x 32 consecutive FP32 columns starting at taddr (one warp).
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
-    uint32_t r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-          "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-          "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
+// 32 lanes x 8 consecutive FP32 columns starting at taddr (one warp).
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                   "=r"(r[7])
+                 : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// The reverse of tmem_ld8 (the caller orders it before later reads).
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float *v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 :
+                 : "r"(taddr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])),
+                   "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])),
+                   "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+                 : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 // Byte offset of element (row, k) in a canonical K-major no-swizzle tile with
@@ -148,67 +155,11 @@ __device__ __forceinline__ uint32_t kmaj_off(int row, int k, int rows) {
     return (uint32_t)((((k >> 3) * (rows >> 3) + (row >> 3)) << 7) + ((row & 7) << 4) + ((k & 7) << 1));
 }
 
-// Run the K/16 MMAs of one tile (A: kRows x K, B: N x K, both canonical) into
-// TMEM and wait.  Thread 0 issues; all threads wait.  Returns false on timeout.
-__device__ __forceinline__ bool umma_tile(const unsigned char *sA, const unsigned char *sB, int K, int N,
-                                          uint32_t taddr, uint64_t *mbar, int *err) {
-    // generic-proxy smem writes -> visible to the tensor-core (async) proxy
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
-        const uint32_t idesc = umma_idesc(N);
-        for (int ks = 0; ks < K / 16; ++ks) {
-            // K slice ks = chunks 2ks, 2ks+1
-            const uint64_t da = umma_desc(a0 + (uint32_t)(2 * ks) * (kRows * 16), kRows * 16, 128);
-            const uint64_t db = umma_desc(b0 + (uint32_t)(2 * ks) * (N * 16), N * 16, 128);
-            umma_f16(taddr, da, db, idesc, ks > 0 ? 1u : 0u);
-        }
-        umma_commit(mbar);
-    }
-    const bool ok = mbar_wait(mbar, 0);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (!ok && threadIdx.x == 0) atomicExch(err, 1);
-    return ok;
-}
-
-// CTA prologue / epilogue: mbarrier + TMEM (warp 0 allocates `ncols`).
-struct TileCtx {
-    uint64_t mbar;
-    uint32_t taddr;
-};
-
-__device__ __forceinline__ void tile_begin(TileCtx *c, int ncols) {
-    if (threadIdx.x == 0) mbar_init(&c->mbar, 1);
-    if (threadIdx.x < 32) tmem_alloc(&c->taddr, ncols);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ void tile_end(TileCtx *c, int ncols, bool ok) {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (!ok) {
-        // the MMAs may still be in flight: one more bounded wait before freeing
-        mbar_wait(&c->mbar, 0);
-    }
-    if (threadIdx.x < 32) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        tmem_dealloc(c->taddr, ncols);
-    }
-}
-
-__device__ __forceinline__ float silu_f(float z) { return z / (1.0f + __expf(-z)); }
-__device__ __forceinline__ float dsilu_f(float z) {
-    const float s = 1.0f / (1.0f + __expf(-z));
-    return s * (1.0f + z * (1.0f - s));
-}
+// SiLU(z) = z s and SiLU'(z) = s (1 + z (1 - s)) from one sigmoid s(z)
+__device__ __forceinline__ float sigmoid_f(float z) { return __frcp_rn(1.0f + __expf(-z)); }
 
 // ---------------------------------------------------------------------------
-// Kernels (128 threads = 4 warps; warp w owns TMEM lanes / rows 32w..32w+31)
+// Kernels
 // ---------------------------------------------------------------------------
 
 // Records -> standardised BF16 inputs X [n x 16] and FP32 targets.
@@ -227,106 +178,351 @@ __global__ void mlp_prepare_kernel(const float *rec, int stride, long long n, co
     T[i] = (r[kIn] - nm.out_mu) * nm.out_isig;
 }
 
-// Z = Hin W^T + b, Hout = SiLU(Z): one 128-row tile per CTA.
-template <int K>
-__global__ void __launch_bounds__(128) mlp_forward_kernel(const bf16 *Hin, const bf16 *W,
-                                                          const float *b, float *Z, bf16 *Hout,
-                                                          long long n, int *err) {
-    __shared__ __align__(128) unsigned char sA[kRows * K * 2];
-    __shared__ __align__(128) unsigned char sB[kH * K * 2];
-    __shared__ TileCtx tc;
-    const long long r0 = (long long)blockIdx.x * kRows;
-    for (int idx = threadIdx.x; idx < kRows * K; idx += blockDim.x) {
-        const int row = idx / K, k = idx % K;
-        const long long g = r0 + row;
-        const bf16 v = g < n ? Hin[g * K + k] : __float2bfloat16_rn(0.0f);
-        *reinterpret_cast<bf16 *>(sA + kmaj_off(row, k, kRows)) = v;
+// The BF16 copies of the weights that the tensor cores read: W [out][in] for
+// the forward products, W^T [in][out] for the data gradients.
+struct Weights {
+    bf16 w1[kH * kInPad], w2[kH * kH], w2t[kH * kH], w3[kH * kH], w3t[kH * kH];
+};
+
+__device__ __forceinline__ void store_bf16(Weights *W, int i, float p) {
+    const bf16 v = __float2bfloat16_rn(p);
+    if (i < kOffB1) {
+        W->w1[i - kOffW1] = v;
+    } else if (i >= kOffW2 && i < kOffB2) {
+        const int q = i - kOffW2;
+        W->w2[q] = v;
+        W->w2t[(q % kH) * kH + q / kH] = v;
+    } else if (i >= kOffW3 && i < kOffB3) {
+        const int q = i - kOffW3;
+        W->w3[q] = v;
+        W->w3t[(q % kH) * kH + q / kH] = v;
     }
-    for (int idx = threadIdx.x; idx < kH * K; idx += blockDim.x) {
-        const int row = idx / K, k = idx % K;
-        *reinterpret_cast<bf16 *>(sB + kmaj_off(row, k, kH)) = W[row * K + k];
+}
+
+__global__ void to_bf16_kernel(const float *P, Weights *W) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kNMaster) store_bf16(W, i, P[i]);
+}
+
+// ---------------------------------------------------------------------------
+// One pass over a batch: forward, output layer, loss and (GRAD) the whole
+// backward pass, or (!GRAD) the predicted levels.
+//
+// A batch of 4096 rows is 0.2 GFLOP: what bounds a training step is not the
+// tensor cores but the number of dependent launches and round trips through
+// memory.  As one kernel per layer and direction, with the activations and
+// pre-activations in global memory and the batch sums in shared-memory
+// atomics, a step took 12 launches and ~450 us.  Here a CTA carries its
+// 128-row tiles through every layer: the pre-activations, and from the forward
+// pass on the SiLU' that the backward pass needs, stay in tensor memory, the
+// activations in shared memory in the two orders the products read them in
+// (K-major by unit for the next layer, K-major by row for the weight
+// gradient), the weight gradients accumulate in tensor memory over the CTA's
+// tiles, and each CTA leaves one row of partial sums that the optimiser adds
+// in a fixed order: 2 launches a step, and a run is reproducible bit for bit.
+//
+// 512 threads: the four warps w, w + 4, ... share the accumulator lanes (rows)
+// 32 (w mod 4) .. + 31 and take 16 columns each.  The element-wise work is one
+// chain of exponential, reciprocal and stores per value: with 8 warps and the
+// column loops unrolled the kernel waited for instructions and latencies (42
+// us a launch at 4096 rows, 15 % issue); 16 warps over rolled loops of 8
+// columns take 23 us (cold caches), the optimiser 6 us.
+// ---------------------------------------------------------------------------
+constexpr int kStepThreads = 512;
+constexpr int kColParts = kStepThreads / kRows;  // threads a row
+// tensor-memory columns
+constexpr int kColZ1 = 0, kColDH = 192, kColW1 = 256, kTmemCols = 512;  // Z and dW: 64 a layer
+
+struct StepSmem {
+    // A operands [128 rows][K] and B operands [N rows][K] of the products
+    alignas(128) unsigned char x[kRows * kInPad * 2];     // A: X, K = inputs
+    alignas(128) unsigned char xt[kInPad * kRows * 2];    // B: X^T, K = rows
+    alignas(128) unsigned char h1[kRows * kH * 2], h2[kRows * kH * 2];     // A, K = units
+    alignas(128) unsigned char h1t[kH * kRows * 2], h2t[kH * kRows * 2];   // B, K = rows
+    alignas(128) unsigned char h3t[kH * kRows * 2];       // H3^T, read by the dw4 sums
+    alignas(128) unsigned char dz[kRows * kH * 2];        // A: dZ, K = units
+    alignas(128) unsigned char dzt[kRows * kRows * 2];    // A: dZ^T, units 64 .. 127 zero, K = rows
+    alignas(128) unsigned char w1[kH * kInPad * 2], w2[kH * kH * 2], w3[kH * kH * 2];
+    alignas(128) unsigned char w2t[kH * kH * 2], w3t[kH * kH * 2];
+    float b[3][kH], w4[kH];
+    float y[kColParts][kRows], gy[kRows], t[kRows];
+    float dw4[kH], db[3][kH], red[2][kStepThreads / 32];
+    uint64_t mbar;
+    uint32_t taddr;
+};
+
+// [N][K] BF16 matrix in global memory -> canonical K-major tile, 16 bytes a thread.
+template <int N, int K>
+__device__ __forceinline__ void stage_weights(unsigned char *dst, const bf16 *src) {
+    for (int c = threadIdx.x; c < N * K / 8; c += kStepThreads) {
+        const int row = c / (K / 8), kc = c % (K / 8);
+        *reinterpret_cast<uint4 *>(dst + kmaj_off(row, 8 * kc, N)) =
+            *reinterpret_cast<const uint4 *>(src + row * K + 8 * kc);
     }
-    tile_begin(&tc, kH);
-    const bool ok = umma_tile(sA, sB, K, kH, tc.taddr, &tc.mbar, err);
-    if (ok) {
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const long long g = r0 + 32 * w + lane;
-        for (int half = 0; half < 2; ++half) {
-            float v[32];
-            tmem_ld32(tc.taddr + ((uint32_t)(32 * w) << 16) + 32 * half, v);
-            if (g < n) {
+}
+
+// Issue the K / 16 MMAs of one product (A: 128 x K, B: N x K, canonical) into
+// the columns at taddr (one thread).
+__device__ __forceinline__ void issue_product(const unsigned char *sA, const unsigned char *sB, int K,
+                                              int N, uint32_t taddr, bool accumulate) {
+    const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
+    const uint32_t idesc = umma_idesc(N);
+#pragma unroll 1
+    for (int ks = 0; ks < K / 16; ++ks) {
+        // K slice ks = chunks 2ks, 2ks+1
+        const uint64_t da = umma_desc(a0 + (uint32_t)(2 * ks) * (kRows * 16), kRows * 16, 128);
+        const uint64_t db = umma_desc(b0 + (uint32_t)(2 * ks) * (N * 16), N * 16, 128);
+        umma_f16(taddr, da, db, idesc, (accumulate || ks > 0) ? 1u : 0u);
+    }
+}
+
+// The CTA's shared-memory operands and tensor-memory reads before this point
+// are visible to the products thread 0 issues after it.
+__device__ __forceinline__ void before_products() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+
+// Eight values of a row, columns col .. col + 7, into a K-major [128][64]
+// tile (kmaj, unless null) and transposed into a [rows_t][128] tile (K = rows).
+__device__ __forceinline__ void put8(unsigned char *kmaj, unsigned char *trans, int rows_t, int row,
+                                     int col, const float *v) {
+    uint4 w;
+    __nv_bfloat162 *p = reinterpret_cast<__nv_bfloat162 *>(&w);
 #pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    const int col = 32 * half + c;
-                    const float z = v[c] + b[col];
-                    Z[g * kH + col] = z;
-                    Hout[g * kH + col] = __float2bfloat16_rn(silu_f(z));
+    for (int c = 0; c < 4; ++c) p[c] = __floats2bfloat162_rn(v[2 * c], v[2 * c + 1]);
+    if (kmaj) *reinterpret_cast<uint4 *>(kmaj + kmaj_off(row, col, kRows)) = w;
+    const bf16 *e = reinterpret_cast<const bf16 *>(&w);
+    unsigned char *t = trans + kmaj_off(col, row, rows_t);  // col is a multiple of 8: 16 bytes a unit
+#pragma unroll
+    for (int c = 0; c < 8; ++c) *reinterpret_cast<bf16 *>(t + 16 * c) = e[c];
+}
+
+// Sum over the tile's rows of unit u of a [rows_t][128] K-major tile (times
+// gy with GY): eight threads a unit, 16 rows each.
+template <bool GY>
+__device__ __forceinline__ float unit_sum(const StepSmem &S, const unsigned char *tile, int rows_t) {
+    const int u = threadIdx.x >> 3, part = threadIdx.x & 7;
+    float acc = 0.0f;
+#pragma unroll 1
+    for (int q = 0; q < 2; ++q) {
+        const int r0 = 16 * part + 8 * q;
+        const uint4 w = *reinterpret_cast<const uint4 *>(tile + kmaj_off(u, r0, rows_t));
+        const bf16 *e = reinterpret_cast<const bf16 *>(&w);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc += GY ? S.gy[r0 + c] * __bfloat162float(e[c]) : __bfloat162float(e[c]);
+    }
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+    return acc;
+}
+
+// perm: row i of the batch is row perm[i] of X and T (null: row i).  part:
+// one row of kPartStride floats per CTA, the gradient in the master layout and
+// the loss after it.  The output layer's weights are rounded to BF16 as in
+// inference; targets are standardised; loss = mean (y - T)^2.
+constexpr int kPartStride = (kNMaster + 1 + 31) / 32 * 32;  // partial rows start on 128 bytes
+template <bool GRAD>
+__global__ void __launch_bounds__(kStepThreads) mlp_step_kernel(const bf16 *X, const float *T,
+                                                                const int *perm, long long n,
+                                                                const Weights *W, const float *P,
+                                                                float *part, float out_mu,
+                                                                float out_sigma, float *y_out,
+                                                                int *err) {
+    extern __shared__ __align__(128) unsigned char step_dyn[];
+    StepSmem &S = *reinterpret_cast<StepSmem *>(step_dyn);
+    const int tid = threadIdx.x, lane = tid & 31, wq = (tid >> 5) & 3, quarter = tid >> 7;
+    const int row = 32 * wq + lane;
+    stage_weights<kH, kInPad>(S.w1, W->w1);
+    stage_weights<kH, kH>(S.w2, W->w2);
+    stage_weights<kH, kH>(S.w3, W->w3);
+    if (GRAD) {
+        stage_weights<kH, kH>(S.w2t, W->w2t);
+        stage_weights<kH, kH>(S.w3t, W->w3t);
+        // dZ^T's units 64 .. 127 and X^T's padding stay zero
+        for (int i = tid; i < kRows * kRows * 2 / 16; i += kStepThreads)
+            reinterpret_cast<uint4 *>(S.dzt)[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = tid; i < kInPad * kRows * 2 / 16; i += kStepThreads)
+            reinterpret_cast<uint4 *>(S.xt)[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (tid < kH) {
+        S.b[0][tid] = P[kOffB1 + tid];
+        S.b[1][tid] = P[kOffB2 + tid];
+        S.b[2][tid] = P[kOffB3 + tid];
+        S.w4[tid] = __bfloat162float(__float2bfloat16_rn(P[kOffW4 + tid]));
+        S.dw4[tid] = S.db[0][tid] = S.db[1][tid] = S.db[2][tid] = 0.0f;
+    }
+    const float b4 = P[kOffB4];
+    if (tid == 0) mbar_init(&S.mbar, 1);
+    if (tid < 32) tmem_alloc(&S.taddr, kTmemCols);
+    before_products();
+    const uint32_t tm = S.taddr;
+    const uint32_t trow = tm + ((uint32_t)(32 * wq) << 16) + 16 * quarter;  // this thread's row and columns
+    const long long tiles = (n + kRows - 1) / kRows;
+    uint32_t phase = 0;
+    bool ok = true;
+    float loss = 0.0f, db4 = 0.0f;
+    // waits for the products committed last; false for every thread of the CTA on a timeout
+    auto wait = [&]() {
+        const bool w = mbar_wait(&S.mbar, phase & 1u);
+        ++phase;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        return __syncthreads_and(w) != 0;
+    };
+    bool first = true;
+    for (long long tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x, first = false) {
+        const long long g = tile * kRows + row;
+        if (quarter == 0) {
+            uint4 a = make_uint4(0u, 0u, 0u, 0u), c = a;
+            float t = 0.0f;
+            if (g < n) {
+                const long long r = perm ? perm[g] : g;
+                const uint4 *src = reinterpret_cast<const uint4 *>(X + r * kInPad);
+                a = src[0];
+                c = src[1];
+                if (GRAD) t = T[r];
+            }
+            *reinterpret_cast<uint4 *>(S.x + kmaj_off(row, 0, kRows)) = a;
+            *reinterpret_cast<uint4 *>(S.x + kmaj_off(row, 8, kRows)) = c;
+            S.t[row] = t;
+            if (GRAD) {
+                const bf16 *e = reinterpret_cast<const bf16 *>(&a);  // columns 8 .. 15 are padding
+#pragma unroll
+                for (int u = 0; u < kIn; ++u)
+                    *reinterpret_cast<bf16 *>(S.xt + kmaj_off(u, row, kInPad)) = e[u];
+            }
+        }
+        // the hidden layers: Z_l stays in tensor memory, H_l goes to shared memory
+        float ys = quarter == 0 ? b4 : 0.0f;
+#pragma unroll 1
+        for (int l = 0; l < 3; ++l) {
+            before_products();
+            if (tid == 0) {
+                issue_product(l == 0 ? S.x : l == 1 ? S.h1 : S.h2, l == 0 ? S.w1 : l == 1 ? S.w2 : S.w3,
+                              l == 0 ? kInPad : kH, kH, tm + kColZ1 + kH * l, false);
+                umma_commit(&S.mbar);
+            }
+            if (!(ok = wait())) break;
+            unsigned char *h = l == 0 ? S.h1 : l == 1 ? S.h2 : nullptr;
+            unsigned char *ht = l == 0 ? S.h1t : l == 1 ? S.h2t : S.h3t;
+#pragma unroll 1
+            for (int q = 0; q < 2; ++q) {
+                const int col = 16 * quarter + 8 * q;
+                float v[8], ds[8];
+                tmem_ld8(trow + kColZ1 + kH * l + 8 * q, v);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const float z = v[c] + S.b[l][col + c], sg = sigmoid_f(z);
+                    v[c] = z * sg;
+                    ds[c] = sg * (1.0f + z * (1.0f - sg));
+                    // the output layer: each thread its columns of the row's dot product
+                    if (l == 2) ys += __bfloat162float(__float2bfloat16_rn(v[c])) * S.w4[col + c];
                 }
+                if (GRAD) tmem_st8(trow + kColZ1 + kH * l + 8 * q, ds);
+                put8(h, ht, kH, row, col, v);
+            }
+        }
+        if (!ok) break;
+        S.y[quarter][row] = ys;
+        __syncthreads();
+        const float y = (S.y[0][row] + S.y[1][row]) + (S.y[2][row] + S.y[3][row]);
+        if constexpr (!GRAD) {
+            if (quarter == 0 && g < n) y_out[g] = y * out_sigma + out_mu;
+        } else {
+            const float d = g < n ? y - S.t[row] : 0.0f;
+            const float gy = 2.0f * d / (float)n;
+            if (quarter == 0) {
+                S.gy[row] = gy;
+                loss += d * d / (float)n;
+                db4 += gy;
+            }
+            // dZ_l, then the products it enters: the weight gradient of layer
+            // l and the data gradient of layer l - 1
+#pragma unroll 1
+            for (int l = 2; l >= 0; --l) {
+#pragma unroll 1
+                for (int q = 0; q < 2; ++q) {
+                    const int col = 16 * quarter + 8 * q;
+                    float ds[8], v[8];
+                    tmem_ld8(trow + kColZ1 + kH * l + 8 * q, ds);
+                    if (l < 2) tmem_ld8(trow + kColDH + 8 * q, v);
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        v[c] = (l == 2 ? gy * S.w4[col + c] : v[c]) * ds[c];
+                    put8(l > 0 ? S.dz : nullptr, S.dzt, kRows, row, col, v);
+                }
+                before_products();
+                if (tid == 0) {
+                    if (l > 0) issue_product(S.dz, l == 2 ? S.w3t : S.w2t, kH, kH, tm + kColDH, false);
+                    issue_product(S.dzt, l == 2 ? S.h2t : l == 1 ? S.h1t : S.xt, kRows, l > 0 ? kH : kInPad,
+                                  tm + kColW1 + kH * l, !first);
+                    umma_commit(&S.mbar);
+                }
+                // while they run: the column sums on the CUDA cores
+                if (l == 2) {
+                    const float dw4 = unit_sum<true>(S, S.h3t, kH);
+                    if ((lane & 7) == 0) S.dw4[tid >> 3] += dw4;
+                }
+                const float db = unit_sum<false>(S, S.dzt, kRows);
+                if ((lane & 7) == 0) S.db[l][tid >> 3] += db;
+                if (!(ok = wait())) break;
             }
         }
     }
-    tile_end(&tc, kH, ok);
-}
-
-// Output layer, loss and its gradient (CUDA cores): y = H3 w4 + b4 with w4
-// rounded to BF16 as in inference (targets standardised), loss = mean (y -
-// T)^2, dZ3 = (2 (y - T) / n) w4 * SiLU'(Z3) stored as BF16 for the
-// tensor-core backward; dw4, db4 accumulated in FP32.  loss receives
-// loss_scale * the batch loss.
-__global__ void mlp_output_kernel(const bf16 *H3, const float *Z3, const float *P, const float *T,
-                                  long long n, bf16 *dZ3, float *G, float *loss, float loss_scale) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    __shared__ float s_w4[kH];
-    __shared__ float s_dw[kH];
-    __shared__ float s_db, s_loss;
-    for (int c = threadIdx.x; c < kH; c += blockDim.x) {
-        s_dw[c] = 0.0f;
-        s_w4[c] = __bfloat162float(__float2bfloat16_rn(P[kOffW4 + c]));
-    }
-    if (threadIdx.x == 0) s_db = s_loss = 0.0f;
-    __syncthreads();
-    if (i < n) {
-        float y = P[kOffB4];
-        for (int c = 0; c < kH; ++c) y += __bfloat162float(H3[i * kH + c]) * s_w4[c];
-        const float d = y - T[i];
-        const float gy = 2.0f * d / (float)n;
-        atomicAdd(&s_loss, d * d / (float)n);
-        atomicAdd(&s_db, gy);
-        for (int c = 0; c < kH; ++c) {
-            atomicAdd(&s_dw[c], gy * __bfloat162float(H3[i * kH + c]));
-            dZ3[i * kH + c] = __float2bfloat16_rn(gy * s_w4[c] * dsilu_f(Z3[i * kH + c]));
+    if constexpr (GRAD) {
+        if (ok) {
+            float *out = part + (size_t)blockIdx.x * kPartStride;
+            // weight gradients: accumulator lane = output unit (64 real), columns = inputs
+            if (wq < 2) {
+#pragma unroll 1
+                for (int q = 0; q < 6; ++q) {
+                    const int l = q >> 1, col = 16 * quarter + 8 * (q & 1), width = l == 0 ? kInPad : kH;
+                    float v[8];
+                    tmem_ld8(trow + kColW1 + kH * l + 8 * (q & 1), v);
+                    if (col < width) {
+                        float *o = out + (l == 0 ? kOffW1 : l == 1 ? kOffW2 : kOffW3) + row * width + col;
+                        *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+                        *reinterpret_cast<float4 *>(o + 4) = make_float4(v[4], v[5], v[6], v[7]);
+                    }
+                }
+            }
+            for (int o = 16; o >= 1; o >>= 1) {
+                loss += __shfl_xor_sync(0xffffffffu, loss, o);
+                db4 += __shfl_xor_sync(0xffffffffu, db4, o);
+            }
+            if (lane == 0) {
+                S.red[0][tid >> 5] = loss;
+                S.red[1][tid >> 5] = db4;
+            }
+            __syncthreads();
+            if (tid < kH) {
+                out[kOffW4 + tid] = S.dw4[tid];
+                out[kOffB1 + tid] = S.db[0][tid];
+                out[kOffB2 + tid] = S.db[1][tid];
+                out[kOffB3 + tid] = S.db[2][tid];
+            }
+            if (tid == 0) {
+                float l = 0.0f, b = 0.0f;
+                for (int w = 0; w < 4; ++w) l += S.red[0][w], b += S.red[1][w];  // quarter 0's warps
+                out[kOffB4] = b;
+                out[kNMaster] = l;
+            }
         }
     }
-    __syncthreads();
-    for (int c = threadIdx.x; c < kH; c += blockDim.x) atomicAdd(&G[kOffW4 + c], s_dw[c]);
-    if (threadIdx.x == 0) {
-        atomicAdd(&G[kOffB4], s_db);
-        if (loss) atomicAdd(loss, s_loss * loss_scale);
+    if (!ok) {
+        // the MMAs may still be in flight: one more bounded wait before freeing
+        if (tid == 0) atomicExch(err, 1);
+        mbar_wait(&S.mbar, (phase + 1u) & 1u);
     }
-}
-
-// Prediction head of the training forward: de-standardised y.
-__global__ void mlp_head_kernel(const bf16 *H3, const float *P, long long n, float out_mu,
-                                float out_sigma, float *y_out) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float y = P[kOffB4];
-    for (int c = 0; c < kH; ++c)
-        y += __bfloat162float(H3[i * kH + c]) * __bfloat162float(__float2bfloat16_rn(P[kOffW4 + c]));
-    y_out[i] = y * out_sigma + out_mu;
-}
-
-// Batch gather: rows perm[0..n) of the prepared inputs and targets.
-__global__ void mlp_gather_kernel(const bf16 *X, const float *T, const int *perm, long long n,
-                                  bf16 *Xb, float *Tb) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const long long r = perm[i];
-    const uint4 *src = reinterpret_cast<const uint4 *>(X + r * kInPad);
-    uint4 *dst = reinterpret_cast<uint4 *>(Xb + i * kInPad);
-    dst[0] = src[0];
-    dst[1] = src[1];
-    Tb[i] = T[r];
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (tid < 32) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_dealloc(tm, kTmemCols);
+    }
 }
 
 // Warp-level inference of the integration kernel on raw feature records.
@@ -344,131 +540,39 @@ __global__ void __launch_bounds__(hhg::kBlockThreads) mlp_infer_kernel(const hhg
     if (i < n) out[i] = T;
 }
 
-// dH = dZ W (W stored [64][K] as W^T [K][64] for this GEMM), then
-// dZprev = dH * SiLU'(Zprev) as BF16 (the first layer has no predecessor).
-template <int K>
-__global__ void __launch_bounds__(128) mlp_backward_data_kernel(const bf16 *dZ, const bf16 *WT,
-                                                                const float *Zprev, bf16 *dZprev,
-                                                                long long n, int *err) {
-    __shared__ __align__(128) unsigned char sA[kRows * kH * 2];
-    __shared__ __align__(128) unsigned char sB[K * kH * 2];
-    __shared__ TileCtx tc;
-    const long long r0 = (long long)blockIdx.x * kRows;
-    for (int idx = threadIdx.x; idx < kRows * kH; idx += blockDim.x) {
-        const int row = idx / kH, k = idx % kH;
-        const long long g = r0 + row;
-        *reinterpret_cast<bf16 *>(sA + kmaj_off(row, k, kRows)) =
-            g < n ? dZ[g * kH + k] : __float2bfloat16_rn(0.0f);
-    }
-    for (int idx = threadIdx.x; idx < K * kH; idx += blockDim.x) {
-        const int row = idx / kH, k = idx % kH;
-        *reinterpret_cast<bf16 *>(sB + kmaj_off(row, k, K)) = WT[row * kH + k];
-    }
-    constexpr int cols = K < 32 ? 32 : K;
-    tile_begin(&tc, cols);
-    const bool ok = umma_tile(sA, sB, kH, K, tc.taddr, &tc.mbar, err);
-    if (ok) {
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const long long g = r0 + 32 * w + lane;
-        for (int half = 0; half < (K + 31) / 32; ++half) {
-            float v[32];
-            tmem_ld32(tc.taddr + ((uint32_t)(32 * w) << 16) + 32 * half, v);
-            if (g < n) {
-#pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    const int col = 32 * half + c;
-                    if (col < K) dZprev[g * K + col] = __float2bfloat16_rn(v[c] * dsilu_f(Zprev[g * K + col]));
-                }
-            }
-        }
-    }
-    tile_end(&tc, cols, ok);
+// Gradient (and loss) = the CTAs' partial rows added in CTA order.
+__device__ __forceinline__ float sum_partials(const float *part, int rows, int i) {
+    float g = 0.0f;
+#pragma unroll 8
+    for (int c = 0; c < rows; ++c) g += part[(size_t)c * kPartStride + i];
+    return g;
 }
 
-// dW [64 x K] += dZ^T Hin over one 64-row chunk: A = dZ^T (64 rows, padded to
-// 128 with zeros), B = Hin^T (K rows), K-dimension = batch rows.
-template <int K>
-__global__ void __launch_bounds__(128) mlp_backward_weight_kernel(const bf16 *dZ, const bf16 *Hin,
-                                                                  long long n, float *dW,
-                                                                  float *db, int *err) {
-    __shared__ __align__(128) unsigned char sA[kRows * kChunk * 2];
-    __shared__ __align__(128) unsigned char sB[K * kChunk * 2];
-    __shared__ TileCtx tc;
-    const long long c0 = (long long)blockIdx.x * kChunk;
-    for (int idx = threadIdx.x; idx < kRows * kChunk; idx += blockDim.x) {
-        const int row = idx / kChunk, kk = idx % kChunk;  // row = output unit, kk = batch row
-        const long long g = c0 + kk;
-        const bf16 v = (row < kH && g < n) ? dZ[g * kH + row] : __float2bfloat16_rn(0.0f);
-        *reinterpret_cast<bf16 *>(sA + kmaj_off(row, kk, kRows)) = v;
-    }
-    for (int idx = threadIdx.x; idx < K * kChunk; idx += blockDim.x) {
-        const int row = idx / kChunk, kk = idx % kChunk;  // row = input unit
-        const long long g = c0 + kk;
-        *reinterpret_cast<bf16 *>(sB + kmaj_off(row, kk, K)) =
-            g < n ? Hin[g * K + row] : __float2bfloat16_rn(0.0f);
-    }
-    // bias gradient: column sums of dZ over the chunk
-    if (threadIdx.x < kH) {
-        float acc = 0.0f;
-        for (int kk = 0; kk < kChunk; ++kk) {
-            const long long g = c0 + kk;
-            if (g < n) acc += __bfloat162float(dZ[g * kH + threadIdx.x]);
-        }
-        atomicAdd(&db[threadIdx.x], acc);
-    }
-    constexpr int cols = K < 32 ? 32 : K;
-    tile_begin(&tc, cols);
-    const bool ok = umma_tile(sA, sB, kChunk, K, tc.taddr, &tc.mbar, err);
-    if (ok) {
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int row = 32 * w + lane;
-        for (int half = 0; half < (K + 31) / 32; ++half) {
-            float v[32];
-            tmem_ld32(tc.taddr + ((uint32_t)(32 * w) << 16) + 32 * half, v);
-            if (row < kH) {
-#pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    const int col = 32 * half + c;
-                    if (col < K) atomicAdd(&dW[row * K + col], v[c]);
-                }
-            }
-        }
-    }
-    tile_end(&tc, cols, ok);
-}
-
-// Adam on the FP32 master parameters, then the BF16 copies.
-__global__ void adam_kernel(float *p, const float *g, float *m, float *v, int n, float lr, float b1,
-                            float b2, float eps, float bc1, float bc2) {
+__global__ void gradient_kernel(const float *part, int rows, float *g) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    m[i] = b1 * m[i] + (1.0f - b1) * gi;
-    v[i] = b2 * v[i] + (1.0f - b2) * gi * gi;
-    p[i] -= lr * (m[i] / bc1) / (sqrtf(v[i] / bc2) + eps);
+    if (i <= kNMaster) g[i] = sum_partials(part, rows, i);
 }
 
-// Master weights -> BF16 W [64][K] and W^T [K][64] of the three hidden
-// layers (one thread per element of all three).
-__global__ void to_bf16_kernel(const float *P, bf16 *W1, bf16 *W2, bf16 *W2T, bf16 *W3, bf16 *W3T) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kH * kInPad) {
-        W1[i] = __float2bfloat16_rn(P[kOffW1 + i]);
+// Adam on the FP32 master parameters from the batch's partial gradients, then
+// the BF16 copies; the thread after the last parameter adds loss_scale x the
+// batch loss to *loss.
+__global__ void adam_kernel(float *p, const float *part, int rows, float *m, float *v, Weights *W,
+                            float lr, float b1, float b2, float eps, float bc1, float bc2,
+                            float *loss, float loss_scale) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > kNMaster) return;
+    const float gi = sum_partials(part, rows, i);
+    if (i == kNMaster) {
+        *loss += gi * loss_scale;
         return;
     }
-    i -= kH * kInPad;
-    if (i < kH * kH) {
-        const bf16 v = __float2bfloat16_rn(P[kOffW2 + i]);
-        W2[i] = v;
-        W2T[(i % kH) * kH + i / kH] = v;
-        return;
-    }
-    i -= kH * kH;
-    if (i < kH * kH) {
-        const bf16 v = __float2bfloat16_rn(P[kOffW3 + i]);
-        W3[i] = v;
-        W3T[(i % kH) * kH + i / kH] = v;
-    }
+    const float mi = b1 * m[i] + (1.0f - b1) * gi;
+    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+    m[i] = mi;
+    v[i] = vi;
+    const float w = p[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+    p[i] = w;
+    store_bf16(W, i, w);
 }
 
 }  // namespace
@@ -539,80 +643,71 @@ uint64_t splitmix64(uint64_t &s) {
     return z ^ (z >> 31);
 }
 
-// Device buffers of one training / evaluation session (freed on scope exit).
+// Device buffers of one training / evaluation session: slices of one
+// allocation (one for each cost 1.0 ms of cudaMalloc and 0.9 ms of cudaFree a
+// call at 262144 records), sized by a first pass over the same requests and freed on scope exit.
 struct Session {
-    std::vector<void *> bufs;
-    cudaError_t err = cudaSuccess;
+    unsigned char *base = nullptr;
+    size_t used = 0;
     template <typename T>
-    T *alloc(size_t n) {
-        void *p = nullptr;
-        if (err == cudaSuccess) err = cudaMalloc(&p, n * sizeof(T) + 16);
-        if (err != cudaSuccess) return nullptr;
-        bufs.push_back(p);
-        return static_cast<T *>(p);
+    void alloc(T *&p, size_t n) {
+        p = base ? reinterpret_cast<T *>(base + used) : nullptr;
+        used += (n * sizeof(T) + 255) / 256 * 256;
     }
-    ~Session() {
-        for (void *p : bufs) cudaFree(p);
+    // `request` names every buffer of the session; it runs twice
+    template <class F>
+    cudaError_t build(F request) {
+        request();
+        const cudaError_t e = cudaMalloc(&base, used);
+        if (e != cudaSuccess) return e;
+        used = 0;
+        request();
+        return cudaSuccess;
     }
+    ~Session() { cudaFree(base); }
 };
 
-// Forward + (optionally) backward buffers for up to `rows` rows.
+// Parameters, their BF16 copies and the partial gradients of one session.
 struct Net {
-    float *P = nullptr, *G = nullptr, *m = nullptr, *v = nullptr;
-    bf16 *W1 = nullptr, *W2 = nullptr, *W2T = nullptr, *W3 = nullptr, *W3T = nullptr;
-    float *Z1 = nullptr, *Z2 = nullptr, *Z3 = nullptr, *Tb = nullptr;
-    bf16 *Xb = nullptr, *H1 = nullptr, *H2 = nullptr, *H3 = nullptr;
-    bf16 *dZ1 = nullptr, *dZ2 = nullptr, *dZ3 = nullptr;
+    float *P = nullptr, *m = nullptr, *v = nullptr, *part = nullptr;
+    Weights *W = nullptr;
     int *err = nullptr;
-    long long rows = 0;
-    bool init(Session &S, long long r, bool optimiser) {
-        rows = (r + kRows - 1) / kRows * kRows;
-        P = S.alloc<float>(kNMaster);
-        G = S.alloc<float>(kNMaster);
+    int max_ctas = 1;
+    cudaError_t init(bool grad) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&max_ctas, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess)
+            e = grad ? cudaFuncSetAttribute(mlp_step_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)sizeof(StepSmem))
+                     : cudaFuncSetAttribute(mlp_step_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)sizeof(StepSmem));
+        return e;
+    }
+    void request(Session &S, bool grad, bool optimiser) {
+        S.alloc(P, kNMaster);
         if (optimiser) {
-            m = S.alloc<float>(kNMaster);
-            v = S.alloc<float>(kNMaster);
+            S.alloc(m, kNMaster);
+            S.alloc(v, kNMaster);
         }
-        W1 = S.alloc<bf16>(kH * kInPad);
-        W2 = S.alloc<bf16>(kH * kH);
-        W2T = S.alloc<bf16>(kH * kH);
-        W3 = S.alloc<bf16>(kH * kH);
-        W3T = S.alloc<bf16>(kH * kH);
-        Xb = S.alloc<bf16>(rows * kInPad);
-        Tb = S.alloc<float>(rows);
-        Z1 = S.alloc<float>(rows * kH);
-        Z2 = S.alloc<float>(rows * kH);
-        Z3 = S.alloc<float>(rows * kH);
-        H1 = S.alloc<bf16>(rows * kH);
-        H2 = S.alloc<bf16>(rows * kH);
-        H3 = S.alloc<bf16>(rows * kH);
-        dZ1 = S.alloc<bf16>(rows * kH);
-        dZ2 = S.alloc<bf16>(rows * kH);
-        dZ3 = S.alloc<bf16>(rows * kH);
-        err = S.alloc<int>(1);
-        return S.err == cudaSuccess;
+        if (grad) S.alloc(part, (size_t)max_ctas * kPartStride);
+        S.alloc(W, 1);
+        S.alloc(err, 1);
+    }
+    // one CTA per SM at most (the step's shared and tensor memory)
+    int ctas(long long n) const {
+        return (int)std::min<long long>((n + kRows - 1) / kRows, max_ctas);
     }
     void weights_bf16(cudaStream_t s) const {
-        const int n = kH * kInPad + 2 * kH * kH;
-        to_bf16_kernel<<<(n + 255) / 256, 256, 0, s>>>(P, W1, W2, W2T, W3, W3T);
+        to_bf16_kernel<<<(kNMaster + 255) / 256, 256, 0, s>>>(P, W);
     }
-    void forward(long long n, cudaStream_t s) const {
-        const unsigned tiles = (unsigned)((n + kRows - 1) / kRows);
-        mlp_forward_kernel<kInPad><<<tiles, 128, 0, s>>>(Xb, W1, P + kOffB1, Z1, H1, n, err);
-        mlp_forward_kernel<kH><<<tiles, 128, 0, s>>>(H1, W2, P + kOffB2, Z2, H2, n, err);
-        mlp_forward_kernel<kH><<<tiles, 128, 0, s>>>(H2, W3, P + kOffB3, Z3, H3, n, err);
+    void gradients(const bf16 *X, const float *T, const int *perm, long long n, cudaStream_t s) const {
+        mlp_step_kernel<true><<<ctas(n), kStepThreads, sizeof(StepSmem), s>>>(X, T, perm, n, W, P, part,
+                                                                              0.0f, 1.0f, nullptr, err);
     }
-    void backward(long long n, float *loss, float loss_scale, cudaStream_t s) const {
-        const unsigned tiles = (unsigned)((n + kRows - 1) / kRows);
-        const unsigned chunks = (unsigned)((n + kChunk - 1) / kChunk);
-        cudaMemsetAsync(G, 0, sizeof(float) * kNMaster, s);
-        mlp_output_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(H3, Z3, P, Tb, n, dZ3, G, loss,
-                                                                      loss_scale);
-        mlp_backward_weight_kernel<kH><<<chunks, 128, 0, s>>>(dZ3, H2, n, G + kOffW3, G + kOffB3, err);
-        mlp_backward_data_kernel<kH><<<tiles, 128, 0, s>>>(dZ3, W3T, Z2, dZ2, n, err);
-        mlp_backward_weight_kernel<kH><<<chunks, 128, 0, s>>>(dZ2, H1, n, G + kOffW2, G + kOffB2, err);
-        mlp_backward_data_kernel<kH><<<tiles, 128, 0, s>>>(dZ2, W2T, Z1, dZ1, n, err);
-        mlp_backward_weight_kernel<kInPad><<<chunks, 128, 0, s>>>(dZ1, Xb, n, G + kOffW1, G + kOffB1, err);
+    void predict(const bf16 *X, long long n, float out_mu, float out_sigma, float *y, cudaStream_t s) const {
+        mlp_step_kernel<false><<<ctas(n), kStepThreads, sizeof(StepSmem), s>>>(
+            X, nullptr, nullptr, n, W, P, nullptr, out_mu, out_sigma, y, err);
     }
 };
 
@@ -642,16 +737,22 @@ hhg_status mlp_train_impl(cudaStream_t s, const float *records, int64_t n, const
     const long long nb = n / B;
     Session S;
     Net W;
-    if (!W.init(S, B, true)) return fail(HHG_CUDA_ERROR, "alloc training buffers", S.err, msg);
-    float *d_rec = S.alloc<float>((size_t)n * HHG_HIST_FIELDS);
-    bf16 *X = S.alloc<bf16>((size_t)n * kInPad);
-    float *T = S.alloc<float>(n);
-    int *perm = S.alloc<int>(n);
-    float *d_loss = S.alloc<float>(o.epochs);
-    if (S.err != cudaSuccess) return fail(HHG_CUDA_ERROR, "alloc training data", S.err, msg);
+    float *d_rec = nullptr, *T = nullptr, *d_loss = nullptr;
+    bf16 *X = nullptr;
+    int *perm = nullptr;
+    cudaError_t e = W.init(true);
+    if (e == cudaSuccess)
+        e = S.build([&] {
+            W.request(S, true, true);
+            S.alloc(d_rec, (size_t)n * HHG_HIST_FIELDS);
+            S.alloc(X, (size_t)n * kInPad);
+            S.alloc(T, (size_t)n);
+            S.alloc(perm, (size_t)n);
+            S.alloc(d_loss, (size_t)o.epochs);
+        });
+    if (e != cudaSuccess) return fail(HHG_CUDA_ERROR, "alloc training buffers", e, msg);
     std::vector<float> master(kNMaster);
     abi_to_master(net->params, master.data());
-    cudaError_t e;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEventCreate(&ev0);
     cudaEventCreate(&ev1);
@@ -674,15 +775,13 @@ hhg_status mlp_train_impl(cudaStream_t s, const float *records, int64_t n, const
         if ((e = cudaMemcpyAsync(perm, hp.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s)) != cudaSuccess)
             return fail(HHG_CUDA_ERROR, "upload batch order", e, msg);
         for (long long b = 0; b < nb; ++b, ++step) {
-            mlp_gather_kernel<<<(unsigned)((B + 255) / 256), 256, 0, s>>>(X, T, perm + b * B, B, W.Xb, W.Tb);
-            W.forward(B, s);
-            W.backward(B, d_loss + ep, 1.0f / (float)nb, s);
+            W.gradients(X, T, perm + b * B, B, s);
             const double t = (double)(step + 1);
             const double lr = o.lr_final + 0.5 * (o.lr - o.lr_final) * (1.0 + std::cos(M_PI * step / total));
-            adam_kernel<<<(kNMaster + 255) / 256, 256, 0, s>>>(
-                W.P, W.G, W.m, W.v, kNMaster, (float)lr, o.beta1, o.beta2, o.eps,
-                (float)(1.0 - std::pow((double)o.beta1, t)), (float)(1.0 - std::pow((double)o.beta2, t)));
-            W.weights_bf16(s);
+            adam_kernel<<<(kNMaster + 1 + 127) / 128, 128, 0, s>>>(
+                W.P, W.part, W.ctas(B), W.m, W.v, W.W, (float)lr, o.beta1, o.beta2, o.eps,
+                (float)(1.0 - std::pow((double)o.beta1, t)), (float)(1.0 - std::pow((double)o.beta2, t)),
+                d_loss + ep, 1.0f / (float)nb);
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return fail(HHG_CUDA_ERROR, "training launch", e, msg);
     }
@@ -713,31 +812,35 @@ hhg_status mlp_gradients_impl(cudaStream_t s, const float *records, int64_t n, c
     if (!check_net(net)) return fail(HHG_BAD_CONFIG, "network standardisation not set", cudaSuccess, msg);
     Session S;
     Net W;
-    if (!W.init(S, n, false)) return fail(HHG_CUDA_ERROR, "alloc buffers", S.err, msg);
-    float *d_rec = S.alloc<float>((size_t)n * HHG_HIST_FIELDS);
-    float *d_loss = S.alloc<float>(1);
-    if (S.err != cudaSuccess) return fail(HHG_CUDA_ERROR, "alloc records", S.err, msg);
-    std::vector<float> master(kNMaster);
+    float *d_rec = nullptr, *T = nullptr, *G = nullptr;  // G: the gradient and the loss
+    bf16 *X = nullptr;
+    cudaError_t e = W.init(true);
+    if (e == cudaSuccess)
+        e = S.build([&] {
+            W.request(S, true, false);
+            S.alloc(d_rec, (size_t)n * HHG_HIST_FIELDS);
+            S.alloc(X, (size_t)n * kInPad);
+            S.alloc(T, (size_t)n);
+            S.alloc(G, kNMaster + 1);
+        });
+    if (e != cudaSuccess) return fail(HHG_CUDA_ERROR, "alloc buffers", e, msg);
+    std::vector<float> master(kNMaster + 1);
     abi_to_master(net->params, master.data());
     cudaMemcpyAsync(d_rec, records, sizeof(float) * n * HHG_HIST_FIELDS, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(W.P, master.data(), sizeof(float) * kNMaster, cudaMemcpyHostToDevice, s);
     cudaMemsetAsync(W.err, 0, sizeof(int), s);
-    cudaMemsetAsync(d_loss, 0, sizeof(float), s);
-    mlp_prepare_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_rec, HHG_HIST_FIELDS, n, make_norm(*net), W.Xb, W.Tb);
+    mlp_prepare_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_rec, HHG_HIST_FIELDS, n, make_norm(*net), X, T);
     W.weights_bf16(s);
-    W.forward(n, s);
-    W.backward(n, d_loss, 1.0f, s);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(HHG_CUDA_ERROR, "gradient launch", e, msg);
+    W.gradients(X, T, nullptr, n, s);
+    gradient_kernel<<<(kNMaster + 1 + 127) / 128, 128, 0, s>>>(W.part, W.ctas(n), G);
+    if ((e = cudaGetLastError()) != cudaSuccess) return fail(HHG_CUDA_ERROR, "gradient launch", e, msg);
     int h_err = 0;
-    float h_loss = 0.0f;
-    cudaMemcpyAsync(master.data(), W.G, sizeof(float) * kNMaster, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(master.data(), G, sizeof(float) * (kNMaster + 1), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(&h_err, W.err, sizeof(int), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&h_loss, d_loss, sizeof(float), cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail(HHG_CUDA_ERROR, "gradients", e, msg);
     if (h_err) return fail(HHG_CUDA_ERROR, "tensor-core completion wait timed out", cudaSuccess, msg);
     master_to_abi(master.data(), grad_out);
-    if (loss_out) *loss_out = h_loss;
+    if (loss_out) *loss_out = master[kNMaster];
     return HHG_OK;
 }
 
@@ -747,15 +850,27 @@ hhg_status mlp_predict_impl(cudaStream_t s, const float *records, int64_t n, con
         return fail(HHG_BAD_CONFIG, "1 <= n_records <= 2^24, path 0 or 1", cudaSuccess, msg);
     if (!check_net(net)) return fail(HHG_BAD_CONFIG, "network standardisation not set", cudaSuccess, msg);
     Session S;
-    float *d_rec = S.alloc<float>((size_t)n * HHG_HIST_FIELDS);
-    float *d_out = S.alloc<float>(n);
-    if (S.err != cudaSuccess) return fail(HHG_CUDA_ERROR, "alloc records", S.err, msg);
+    Net W;
+    float *d_rec = nullptr, *d_out = nullptr, *T = nullptr;
+    bf16 *X = nullptr;
+    MlpPacked *d_net = nullptr;
+    cudaError_t e = path == 1 ? W.init(false) : cudaSuccess;
+    if (e == cudaSuccess)
+        e = S.build([&] {
+            S.alloc(d_rec, (size_t)n * HHG_HIST_FIELDS);
+            S.alloc(d_out, (size_t)n);
+            if (path == 0) {
+                S.alloc(d_net, 1);
+            } else {
+                W.request(S, false, false);
+                S.alloc(X, (size_t)n * kInPad);
+                S.alloc(T, (size_t)n);
+            }
+        });
+    if (e != cudaSuccess) return fail(HHG_CUDA_ERROR, "alloc buffers", e, msg);
     cudaMemcpyAsync(d_rec, records, sizeof(float) * n * HHG_HIST_FIELDS, cudaMemcpyHostToDevice, s);
     int h_err = 0;
-    Net W;
     if (path == 0) {
-        MlpPacked *d_net = S.alloc<MlpPacked>(1);
-        if (S.err != cudaSuccess) return fail(HHG_CUDA_ERROR, "alloc network", S.err, msg);
         MlpPacked h;
         pack_mlp(*net, &h);
         cudaMemcpyAsync(d_net, &h, sizeof h, cudaMemcpyHostToDevice, s);
@@ -763,22 +878,18 @@ hhg_status mlp_predict_impl(cudaStream_t s, const float *records, int64_t n, con
         mlp_infer_kernel<<<(unsigned)((n + rows_per_cta - 1) / rows_per_cta), kBlockThreads, mlp_smem_bytes(), s>>>(
             d_net, d_rec, HHG_HIST_FIELDS, n, d_out);
         // the packed copy must outlive the kernel: synchronise before the session frees it
-        cudaError_t e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return fail(HHG_CUDA_ERROR, "inference", e, msg);
+        if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail(HHG_CUDA_ERROR, "inference", e, msg);
     } else {
-        if (!W.init(S, n, false)) return fail(HHG_CUDA_ERROR, "alloc buffers", S.err, msg);
         std::vector<float> master(kNMaster);
         abi_to_master(net->params, master.data());
         cudaMemcpyAsync(W.P, master.data(), sizeof(float) * kNMaster, cudaMemcpyHostToDevice, s);
         cudaMemsetAsync(W.err, 0, sizeof(int), s);
-        mlp_prepare_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_rec, HHG_HIST_FIELDS, n, make_norm(*net), W.Xb, W.Tb);
+        mlp_prepare_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_rec, HHG_HIST_FIELDS, n, make_norm(*net), X, T);
         W.weights_bf16(s);
-        W.forward(n, s);
-        mlp_head_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(W.H3, W.P, n, net->out_mu, net->out_sigma, d_out);
+        W.predict(X, n, net->out_mu, net->out_sigma, d_out, s);
         cudaMemcpyAsync(&h_err, W.err, sizeof(int), cudaMemcpyDeviceToHost, s);
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(HHG_CUDA_ERROR, "predict launch", e, msg);
+    if ((e = cudaGetLastError()) != cudaSuccess) return fail(HHG_CUDA_ERROR, "predict launch", e, msg);
     cudaMemcpyAsync(out, d_out, sizeof(float) * n, cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail(HHG_CUDA_ERROR, "predict", e, msg);
     if (h_err) return fail(HHG_CUDA_ERROR, "tensor-core completion wait timed out", cudaSuccess, msg);
