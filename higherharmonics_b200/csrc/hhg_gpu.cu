@@ -1488,8 +1488,10 @@ hhg_status enqueue_integration(hhg_plan *pl, cudaStream_t s, bool events) {
     lr.kp.max_failed = pl->opts.max_failed_steps;
     lr.kp.max_attempts = pl->opts.max_attempts_per_interval;
     lr.kp.magnus_substeps = pl->opts.magnus_substeps;
-    lr.kp.abs_tol = pl->opts.abs_tol;
-    lr.kp.rel_tol = pl->opts.rel_tol;
+    const double tol_scale =
+        hhg::scaled_attempt(pl->model, pl->opts.precision == HHG_PREC_FP64) ? hhg::kErrScale : 1.0;
+    lr.kp.abs_tol = pl->opts.abs_tol * tol_scale;
+    lr.kp.rel_tol = pl->opts.rel_tol * tol_scale;
     lr.kp.err_floor = pow(5.0, -8.0);
     lr.kp.grow_max = 9.0 / 10.0 * pow(pow(5.0, -8.0), -1.0 / 8);
     lr.kp.mlp = pl->d_mlp;

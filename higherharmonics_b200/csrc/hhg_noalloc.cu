@@ -326,8 +326,10 @@ extern "C" hhg_status hhg_gpu_current_density_noalloc(const hhg_system_desc *sys
     lr.kp.max_failed = o.max_failed_steps;
     lr.kp.max_attempts = o.max_attempts_per_interval;
     lr.kp.magnus_substeps = o.magnus_substeps;
-    lr.kp.abs_tol = o.abs_tol;
-    lr.kp.rel_tol = o.rel_tol;
+    const double tol_scale =
+        hhg::scaled_attempt(prep.model, o.precision == HHG_PREC_FP64) ? hhg::kErrScale : 1.0;
+    lr.kp.abs_tol = o.abs_tol * tol_scale;
+    lr.kp.rel_tol = o.rel_tol * tol_scale;
     lr.kp.err_floor = pow(5.0, -8.0);
     lr.kp.grow_max = grow_max;
     lr.kp.coarsen = 1.0 / hhg::kCoarsenDivFp64;  // dyadic stepping only; not offered here
