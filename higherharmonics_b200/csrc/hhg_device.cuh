@@ -74,14 +74,12 @@ __host__ __device__ constexpr int base_model(int m) {
 // Number of staged pulse functions per model: A for the Dirac models, (cos,
 // sin) pairs of s A(t) for the lattice models.  kRelax: FP64 RKF78 only.
 // kStart: the right-hand side also reads the step's start state.
-// kMinBlocks: integration CTAs per SM the register budget is sized for.
 // kPacked: the FP32 right-hand side runs on packed (x, y) pairs (rhs2).
 // kPairs: the FP32 staged values of the two projections are interleaved
 // (below, pair_layout), so rhs2 takes them as packed operands without moves.
 template <int M> struct Traits {
     static constexpr bool kRelax = false;
     static constexpr bool kStart = false;
-    static constexpr int kMinBlocks = kMinBlocksPerSM;
     static constexpr bool kPacked = false;
     static constexpr bool kPairs = false;
     static constexpr bool kHiFirst = false;
@@ -111,9 +109,6 @@ template <> struct Traits<PIFLUX3D_RELAX> {
     static constexpr int NF = 2;
     static constexpr bool kRelax = true;
     static constexpr bool kStart = true;
-    // 255 registers, 8 warps per SM: at 168 registers (12 warps) the stage
-    // values spill and the kernel runs 1.7x slower (measured)
-    static constexpr int kMinBlocks = 4;
 };
 template <> struct Traits<HONEYCOMB_RELAX> {
     static constexpr bool kPairs = false;
@@ -121,7 +116,6 @@ template <> struct Traits<HONEYCOMB_RELAX> {
     static constexpr int NF = 6;
     static constexpr bool kRelax = true;
     static constexpr bool kStart = false;
-    static constexpr int kMinBlocks = 4;  // 255 registers: the six staged functions spill at 168
 };
 template <> struct Traits<DIRAC3D_RELAX> {
     static constexpr bool kPairs = false;
@@ -129,7 +123,6 @@ template <> struct Traits<DIRAC3D_RELAX> {
     static constexpr int NF = 1;
     static constexpr bool kRelax = true;
     static constexpr bool kStart = false;
-    static constexpr int kMinBlocks = kMinBlocksPerSM;
 };
 
 // Whether the model's RKF78 attempts run in the scaled form (stages h k): all
@@ -143,7 +136,7 @@ __host__ __device__ constexpr bool scaled_attempt(int model, bool fp64) {
 //   [5, 5+nf) the staged functions evaluated exactly at the interval's end
 //   sample t_s = (i+1) * measure_every + window_begin        (header, even)
 //   nf * (deg + 1) monomial coefficients                        (poly)
-//   [n_std, pad, ts[kMaxStd], hs[kMaxStd]]                      (schedule)
+//   [n_std, error bound of step n_std - 2, ts[kMaxStd], hs[kMaxStd]]  (schedule)
 //   kMaxStd x 13 x nf exact stage values                        (table)
 __host__ __device__ constexpr int slot_header(int nf) { return (5 + nf + 1) & ~1; }
 __host__ __device__ constexpr int slot_poly(int nf) { return slot_header(nf); }
@@ -1459,18 +1452,23 @@ __device__ __forceinline__ double error_den(const KParams &P, double S, double k
 // default error checker and step adjuster).  Returns true if accepted and
 // updates dt.  err < 5^-8 takes the host-computed growth constant;
 // the mixed-precision variant evaluates the power of the growth/shrink factor
-// in FP32.
+// in FP32.  LAST: an accepted step ends the interval and nothing reads the
+// grown dt (every interval restarts at dt0), so an accepted step needs neither
+// the quotients nor the power (~200 FP64 instructions at the end of every
+// interval, where the clipped step's error is above 5^-8 as a rule).
 template <int M, typename R>
 __device__ __forceinline__ bool control(const KParams &P, const double *S, const double *e,
-                                        const double *k0, double &dt) {
+                                        const double *k0, double &dt, bool last = false) {
     constexpr bool FAST_POW = sizeof(R) != sizeof(double);
     double den[3];
-    bool tiny = true;
+    bool tiny = true, pass = true;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         den[c] = error_den<M, R>(P, S[c], k0[c], dt);
         tiny = tiny && (fabs(e[c]) < P.err_floor * den[c]);
+        pass = pass && (fabs(e[c]) < den[c]);
     }
+    if (last && pass) return true;
     if (tiny) {
         dt *= P.grow_max;
         return true;
@@ -1497,8 +1495,20 @@ __device__ __forceinline__ bool control(const KParams &P, const double *S, const
 // clip the step to land on t1; loop while t1 - t > DBL_EPSILON; err =
 // max_i |e_i| / (abs + rel (|x_i| + dt |dxdt_i|)); err > 1: dt *= max(0.9
 // err^-1/6, 0.2) and retry; else accept and, if err < 0.5, dt *= 0.9 max(err,
-// 5^-8)^-1/8.  With USE_STD the warp reads the tabulated pulse values while all
-// active lanes are on the standard schedule.  Called by the whole warp.
+// 5^-8)^-1/8.  Called by the whole warp.
+//
+// USE_STD: the interval starts on the standard schedule (t = t0, dt = dt0),
+// and stays on it while every lane's error is below 5^-8 (for the step before
+// the clipped last one below the staged bound that still reaches t1, for the
+// last one below 1).  There the step is the schedule's for the
+// whole warp: pulse values from the table, no per-lane t and dt, and one vote
+// an attempt.  The first attempt that takes a lane off the schedule is
+// finished by the per-lane controller, which then goes on with the
+// interpolants.  Before, every lane ran its own controller on the table path
+// too: votes on t and dt, and at the ends of the third and fourth step of an
+// interval three quotients and a power.  With the records one interval ahead
+// and the samples summed in blocks: pi-flux 256 x 256 (8192 intervals) 76.6 ->
+// 54.6 ms, gapped Dirac 64 x 64 14.0 -> 9.3 ms.
 // ---------------------------------------------------------------------------
 template <int M, int NF, int D, typename R, bool USE_STD, bool CARRY, bool REC = false>
 __device__ __forceinline__ void lane_controller(const KParams &P, const ModelState<M, R> &ms,
@@ -1512,79 +1522,107 @@ __device__ __forceinline__ void lane_controller(const KParams &P, const ModelSta
                                                 const PulseDev *pd = nullptr,
                                                 bool rec_lane = false) {
     constexpr int SCHED = slot_sched(NF, D);
-    bool active = !dead;
-    int fails = 0, attempts = 0, wa = 0;
-    while (__any_sync(kFull, active)) {
-        if (active && (t + dt) - t1 > kDblEps) dt = t1 - t;
-        bool table = false;
-        if constexpr (USE_STD) {
-            // every active lane on the standard schedule -> table path
-            const bool on = !active || (wa < n_std && t == slot[SCHED + 2 + wa] &&
-                                        dt == slot[SCHED + 2 + kMaxStd + wa]);
-            table = __all_sync(kFull, on);
+    const bool alive = !dead;
+    bool active = alive;
+    int fails = 0, attempts = 0;
+    // this lane's outcome of an attempt of size dt from t
+    auto finish = [&](const double *xn, const double *e, const double *k0) {
+        ++attempts;
+        const double dt_used = dt;
+        if (REC && rec_lane && attempts == 1) {
+            // accept/reject history of the interval's first attempt:
+            // features, and the level T = log2(span / h*) of the largest
+            // step with err <= 0.9, h* = h (0.9 / err)^(1/8)
+            double err = 0.0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                err = fmax(err, fabs(e[c]) / error_den<M, R>(P, S[c], k0[c], dt));
+            const double span = slot[1] - slot[0];
+            double T = log2(span / dt_used) - (err > 0.0 ? 0.125 * log2(0.9 / err) : 64.0);
+            T = fmin(fmax(T, -1.0), 12.0);
+            const unsigned long long at = atomicAdd(P.hist_count, 1ull);
+            if ((long long)at < P.hist_cap) {
+                float f[kMlpIn];
+                mlp_features(mlp_k_features(row), laser_exact(*pd, t), laser_field(*pd, t), S,
+                             log2(dt_used / span), f);
+                float *o = P.hist + (size_t)at * kHistFields;
+#pragma unroll
+                for (int c = 0; c < kMlpIn; ++c) o[c] = f[c];
+                o[8] = float(T);
+                o[9] = float(dt_used / span);
+                o[10] = float(err);
+                o[11] = 0.0f;
+            }
         }
-        if (active) {
-            double xn[3], e[3], k0[3];
-            if (table) {
-                const TableEval<NF, R, table_values<M, R>()> tev{tabv + wa * 13 * NF};
-                rkf78_attempt<M, NF, R>(ms, tev, t, dt, S, xn, e, k0);
-            } else {
-                rkf78_attempt<M, NF, R>(ms, poly, t, dt, S, xn, e, k0);
-            }
-            ++attempts;
-            const double dt_used = dt;
-            if (REC && rec_lane && attempts == 1) {
-                // accept/reject history of the interval's first attempt:
-                // features, and the level T = log2(span / h*) of the largest
-                // step with err <= 0.9, h* = h (0.9 / err)^(1/8)
-                double err = 0.0;
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    err = fmax(err, fabs(e[c]) / error_den<M, R>(P, S[c], k0[c], dt));
-                const double span = slot[1] - slot[0];
-                double T = log2(span / dt_used) - (err > 0.0 ? 0.125 * log2(0.9 / err) : 64.0);
-                T = fmin(fmax(T, -1.0), 12.0);
-                const unsigned long long at = atomicAdd(P.hist_count, 1ull);
-                if ((long long)at < P.hist_cap) {
-                    float f[kMlpIn];
-                    mlp_features(mlp_k_features(row), laser_exact(*pd, t), laser_field(*pd, t), S,
-                                 log2(dt_used / span), f);
-                    float *o = P.hist + (size_t)at * kHistFields;
-#pragma unroll
-                    for (int c = 0; c < kMlpIn; ++c) o[c] = f[c];
-                    o[8] = float(T);
-                    o[9] = float(dt_used / span);
-                    o[10] = float(err);
-                    o[11] = 0.0f;
-                }
-            }
-            if (control<M, R>(P, S, e, k0, dt)) {
-                t += dt_used;
-                S[0] = xn[0];
-                S[1] = xn[1];
-                S[2] = xn[2];
-                fails = 0;
-                if (!(t1 - t > kDblEps)) active = false;
-                if (CARRY) carry_dt = dt;
-            } else {
-                ++rejects;
-                if (++fails >= P.max_failed) {
-                    active = false;
-                    dead = true;
-                    atomicAdd(P.counters + 3, 1ull);
-                    atomicMax(P.status, 2);
-                }
-            }
-            if (active && attempts >= P.max_attempts) {
+        if (control<M, R>(P, S, e, k0, dt, !CARRY && !(t1 - (t + dt_used) > kDblEps))) {
+            t += dt_used;
+            S[0] = xn[0];
+            S[1] = xn[1];
+            S[2] = xn[2];
+            fails = 0;
+            if (!(t1 - t > kDblEps)) active = false;
+            if (CARRY) carry_dt = dt;
+        } else {
+            ++rejects;
+            if (++fails >= P.max_failed) {
                 active = false;
                 dead = true;
                 atomicAdd(P.counters + 3, 1ull);
                 atomicMax(P.status, 2);
             }
         }
-        ++wa;
+        if (active && attempts >= P.max_attempts) {
+            active = false;
+            dead = true;
+            atomicAdd(P.counters + 3, 1ull);
+            atomicMax(P.status, 2);
+        }
+    };
+    if constexpr (USE_STD) {
+#pragma unroll 1
+        for (int wa = 0; wa < n_std; ++wa) {
+            t = slot[SCHED + 2 + wa];
+            dt = slot[SCHED + 2 + kMaxStd + wa];
+            const TableEval<NF, R, table_values<M, R>()> tev{tabv + wa * 13 * NF};
+            double xn[3], e[3], k0[3];
+            rkf78_attempt<M, NF, R>(ms, tev, t, dt, S, xn, e, k0);
+            const bool last = !(t1 - (t + dt) > kDblEps);
+            const double floor = last ? 1.0 : wa == n_std - 2 ? slot[SCHED + 1] : P.err_floor;
+            bool on = true;
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                on = on && (fabs(e[c]) < floor * error_den<M, R>(P, S[c], k0[c], dt));
+            if (!__all_sync(kFull, on || !active) || (!last && wa + 1 >= P.max_attempts)) {
+                if (active) finish(xn, e, k0);
+                break;
+            }
+            ++attempts;
+            if (active) {
+                S[0] = xn[0];
+                S[1] = xn[1];
+                S[2] = xn[2];
+            }
+            if (last) active = false;
+            t += dt;
+            dt *= P.grow_max;
+        }
     }
-    attempts_out += attempts;
+    while (__any_sync(kFull, active)) {
+        if (active) {
+            if ((t + dt) - t1 > kDblEps) dt = t1 - t;
+            double xn[3], e[3], k0[3];
+            rkf78_attempt<M, NF, R>(ms, poly, t, dt, S, xn, e, k0);
+            finish(xn, e, k0);
+        }
+    }
+    if (alive) attempts_out += attempts;
+}
+
+__device__ __forceinline__ void copy16_async(void *smem, const void *gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                 :
+                 : "r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -1623,6 +1661,34 @@ __device__ __forceinline__ void lane_controller(const KParams &P, const ModelSta
 // ends.
 // ---------------------------------------------------------------------------
 constexpr int kFreeWindow = 8;
+
+// Samples of the interval-synchronous loop: the lanes' weighted currents of
+// eight consecutive samples wait in a per-warp block of shared memory and are
+// summed together, lane (s, part) = (lane mod 8, lane / 8) taking eight lanes
+// of sample s, then two shuffles over the parts: 1 + 10/8 shared-memory
+// operations and 1.5 FP64 additions a sample, off the step chain, where a
+// butterfly per sample costs ten shuffles and five additions in a row (175
+// cycles).  A fixed order.  Rows are padded to 33 doubles (bank conflicts).
+constexpr int kRing = 8, kRingRow = 33;
+__device__ __forceinline__ void put_sample(int i, double c, int N, int sub, int lane, double *ring,
+                                           double *prow) {
+    ring[(i & (kRing - 1)) * kRingRow + lane] = c;
+    if ((i & (kRing - 1)) != kRing - 1 && i != N) return;
+    __syncwarp();
+    const int s = lane & (kRing - 1), part = lane / kRing;
+    const double *r = ring + s * kRingRow + part * (32 / 4);
+    double v = 0.0;
+#pragma unroll
+    for (int k = 0; k < 32 / 4; ++k) v += r[k];
+    v += __shfl_xor_sync(kFull, v, 8);
+    v += __shfl_xor_sync(kFull, v, 16);
+    const int at = (i & ~(kRing - 1)) + s;
+    if (part == 0 && at <= i) {
+        if (sub == 0) prow[at] = v;
+        else prow[at] += v;
+    }
+    __syncwarp();
+}
 
 // Sample i's warp sum: lane i mod 32 keeps it; every 32 samples (and at the
 // last) one coalesced store (or accumulation, for later k tiles of the item).
@@ -1665,7 +1731,7 @@ __device__ void integrate_free(const KParams &P, const PulseDev &pd, const Model
                 ++attempts;
                 ++attempts_out;
                 const double dt_used = dt;
-                if (control<M, double>(P, S, e, k0, dt)) {
+                if (control<M, double>(P, S, e, k0, dt, !(t1 - (t + dt_used) > kDblEps))) {
                     t += dt_used;
                     S[0] = xn[0];
                     S[1] = xn[1];
@@ -1736,6 +1802,19 @@ __host__ __device__ constexpr int mlp_smem_bytes() { return mlp_stage_bytes(kWar
 constexpr int kCoarsenDivFp64 = 600;
 constexpr int kCoarsenDivMixed = 64;
 
+// Integration CTAs per SM the register budget of a variant is sized for.
+// FP64 RKF78: 5 (168 registers, up to 3 warps per scheduler).  One warp's
+// attempt keeps the FP64 pipe 80 % busy, so registers without spills are
+// worth more than a fourth warp: 7 -> 5 CTAs, honeycomb 512 x 512 8.08 ->
+// 7.35 ms (256 intervals), pi-flux 256 x 256 3.47 -> 3.37 ms (512 intervals).
+// The lattice models' relaxation: 4 (255 registers; at 168 the stage values
+// spill, 1.7x slower).
+__host__ __device__ constexpr int min_blocks(int model, bool fp64, int stepper) {
+    return fp64 && stepper == 0 && model != PIFLUX3D_RELAX && model != HONEYCOMB_RELAX ? 5
+           : model == PIFLUX3D_RELAX || model == HONEYCOMB_RELAX                       ? 4
+                                                                                       : kMinBlocksPerSM;
+}
+
 // OUT 0: the Brillouin-zone sum of the current (one partial row per item);
 // OUT 1: the same split by the instantaneous energy |d(k - A(t_i))| < energy_cut
 //   into two channels (PiFlux::current_per_energy, PiFlux.cpp:955-1035);
@@ -1748,7 +1827,8 @@ constexpr int kCoarsenDivMixed = 64;
 //   DiracSystem.cpp:300-311; dead trajectories give 0 and are counted).
 // OUT 1-3 are built for the PiFlux models only, OUT 4 for the Dirac-3D ones.
 template <int M, int D, typename R, int STEPPER, int PROPOSER, int OUT = 0>
-__global__ void __launch_bounds__(kBlockThreads, Traits<M>::kMinBlocks) bz_integrate_kernel(const KParams P) {
+__global__ void __launch_bounds__(kBlockThreads, min_blocks(M, sizeof(R) == sizeof(double), STEPPER))
+bz_integrate_kernel(const KParams P) {
     constexpr int NF = Traits<M>::NF;
     constexpr bool kDyadic = PROPOSER == 2 || PROPOSER == 3;
     constexpr bool kLearned = PROPOSER == 3;
@@ -1767,8 +1847,13 @@ __global__ void __launch_bounds__(kBlockThreads, Traits<M>::kMinBlocks) bz_integ
     constexpr int COPY = kFree ? 2 : (PROPOSER == 0) ? SLOT : SCHED;
     constexpr int NTAB = kMaxStd * 13 * NF;
     using V = typename Num<R>::V;
-    __shared__ __align__(16) double stage_raw[kWarpsPerBlock][COPY];
+    // FP64 RKF78: interval records are copied one interval ahead (cp.async) into
+    // two buffers, and samples are summed eight at a time (put_sample)
+    constexpr bool kFetch = STEPPER == 0 && !kNarrow && !kFree;
+    __shared__ __align__(16) double stage_raw[kWarpsPerBlock][kFetch ? 2 : 1][COPY];
     __shared__ double free_ring[kWarpsPerBlock][kFree ? kFreeWindow * 32 : 1];
+    constexpr bool kRingSum = STEPPER == 0 && !kNarrow && !kFree && OUT == 0;
+    __shared__ double ring[kWarpsPerBlock][kRingSum ? kRing * kRingRow : 1];
     __shared__ __align__(16) V stage_tab[kWarpsPerBlock][kNarrow && PROPOSER == 0 ? NTAB : 1];
     // learned proposer: per-warp input tiles in dynamic shared memory
     // (mlp_smem_bytes(); none for the other modes); the network itself is
@@ -1777,10 +1862,7 @@ __global__ void __launch_bounds__(kBlockThreads, Traits<M>::kMinBlocks) bz_integ
     __nv_bfloat16 *mlp_stage = reinterpret_cast<__nv_bfloat16 *>(dyn_smem);
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    double *slot = stage_raw[wib];
-    const V *tabv;
-    if constexpr (kNarrow && PROPOSER == 0) tabv = stage_tab[wib];
-    else tabv = reinterpret_cast<const V *>(slot + (PROPOSER == 0 ? TAB : 0));
+    double *slot = stage_raw[wib][0];
 
     unsigned long long my_attempts = 0, my_rejects = 0;
     for (;;) {
@@ -1839,6 +1921,17 @@ __global__ void __launch_bounds__(kBlockThreads, Traits<M>::kMinBlocks) bz_integ
                 for (int c = 0; c < 4; ++c) mom_next[c] = __ldg(coef + TAB + c);
             }
 
+            auto fetch = [&](int interval) {
+                const double *src = coef + (size_t)interval * SLOT;
+                double *dst = stage_raw[wib][interval & (kFetch ? 1 : 0)];
+                for (int c = lane; c < COPY / 2; c += 32) copy16_async(dst + 2 * c, src + 2 * c);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            };
+            if constexpr (kFetch) {
+                __syncwarp();  // the previous tile's last record has been read
+                fetch(0);
+            }
+
             if constexpr (kFree) {
                 // sample 0 at t_begin, then free lanes through samples 1 .. N
                 keep_sample(0, warp_sum(dead ? 0.0 : w * ms.vertex(pd.s0rec, S)), N, sub, lane, held,
@@ -1849,19 +1942,31 @@ __global__ void __launch_bounds__(kBlockThreads, Traits<M>::kMinBlocks) bz_integ
             for (int i = 0; i <= N; ++i) {
                 const double *rec = pd.s0rec;
                 if (i > 0) {
-                    // stage interval i-1 into this warp's shared slot (the
-                    // Magnus steppers read their interpolants or moments and
-                    // the record straight from the staging table: warp
-                    // broadcasts of a few values per interval)
+                    // interval i-1 in this warp's shared slot (the Magnus
+                    // steppers read their interpolants or moments and the
+                    // record straight from the staging table: warp broadcasts
+                    // of a few values per interval)
                     const double *gslot = coef + (size_t)(i - 1) * SLOT;
-                    if constexpr (STEPPER == 0) {
+                    if constexpr (kFetch) {
+                        slot = stage_raw[wib][(i - 1) & 1];
+                        __syncwarp();  // the other buffer has been read
+                        if (i < N) {
+                            fetch(i);
+                            asm volatile("cp.async.wait_group 1;" ::: "memory");
+                        } else {
+                            asm volatile("cp.async.wait_group 0;" ::: "memory");
+                        }
+                        __syncwarp();
+                    } else if constexpr (STEPPER == 0) {
                         __syncwarp();
                         const double2 *src = reinterpret_cast<const double2 *>(gslot);
                         double2 *dst = reinterpret_cast<double2 *>(slot);
                         for (int c = lane; c < COPY / 2; c += 32) dst[c] = __ldg(src + c);
-                    }
-                    if constexpr (kNarrow && PROPOSER == 0) {
                         __syncwarp();
+                    }
+                    const V *tabv = reinterpret_cast<const V *>(slot + (PROPOSER == 0 ? TAB : 0));
+                    if constexpr (kNarrow && PROPOSER == 0) tabv = stage_tab[wib];
+                    if constexpr (kNarrow && PROPOSER == 0) {
                         for (int c = lane; c < NTAB; c += 32) {
                             if constexpr (kPair)
                                 stage_tab[wib][c] =
@@ -1869,8 +1974,8 @@ __global__ void __launch_bounds__(kBlockThreads, Traits<M>::kMinBlocks) bz_integ
                             else
                                 stage_tab[wib][c] = Num<R>::mk(slot[TAB + c]);
                         }
+                        __syncwarp();
                     }
-                    __syncwarp();
                     const double *cur = STEPPER != 0 ? gslot : slot;
                     rec = cur + 4;
                     const double t0 = cur[0], t1 = cur[1];
@@ -1942,11 +2047,11 @@ __global__ void __launch_bounds__(kBlockThreads, Traits<M>::kMinBlocks) bz_integ
                         // every lane records every hist_every-th interval, staggered
                         const bool rec_lane =
                             kRecord && ((i - 1 + lane + (int)(item & 1023)) % P.hist_every) == 0;
-                        // the relaxation models' steps follow their dynamics, not the
+                        // the lattice models' relaxation steps follow their dynamics, not the
                         // standard schedule; without the table path their attempt code is
                         // half the size (5 % faster, measured)
-                        lane_controller<M, NF, D, R, PROPOSER == 0 && !Traits<M>::kRelax, kCarry,
-                                        kRecord>(
+                        lane_controller<M, NF, D, R, PROPOSER == 0 && (!Traits<M>::kRelax || M == DIRAC3D_RELAX),
+                                        kCarry, kRecord>(
                             P, ms, poly, slot, tabv, n_std, t0, kCarry ? carry_dt : dt0,
                             t1, S, dead, carry_dt, my_attempts, my_rejects, row, &pd, rec_lane);
                     } else {
@@ -2040,17 +2145,8 @@ __global__ void __launch_bounds__(kBlockThreads, Traits<M>::kMinBlocks) bz_integ
                 // sample i at t_i = i * measure_every + t_begin (PiFlux.cpp:834-836)
                 if constexpr (OUT == 0) {
                     const double c = dead ? 0.0 : w * ms.vertex(rec, S);
-                    const double sum = warp_sum(c);
-                    if (lane == (i & 31)) held = sum;
-                    if ((i & 31) == 31 || i == N) {
-                        const int base = i & ~31;
-                        if (base + lane <= N) {
-                            if (sub == 0)
-                                prow[base + lane] = held;
-                            else
-                                prow[base + lane] += held;
-                        }
-                    }
+                    if constexpr (kRingSum) put_sample(i, c, N, sub, lane, ring[wib], prow);
+                    else keep_sample(i, warp_sum(c), N, sub, lane, held, prow);
                 } else if constexpr (OUT == 1) {
                     double c_lo = 0.0, c_hi = 0.0;
                     if (!dead) {
@@ -2122,7 +2218,8 @@ __global__ void stage_pulses_kernel(const PulseDev *__restrict__ pulses, int n_p
                                     const double *__restrict__ tgrid,
                                     const long long *__restrict__ interval_off,
                                     double *__restrict__ coef, long long total_intervals,
-                                    double grow_max, const double *__restrict__ gl30) {
+                                    double grow_max, double err_floor,
+                                    const double *__restrict__ gl30) {
     constexpr int NF = Traits<M>::NF;
     constexpr int SLOT = (LAYOUT == 0 || LAYOUT == 3) ? slot_doubles(NF, D) : slot_doubles_dyadic(NF, D);
     constexpr int HDR = slot_header(NF);
@@ -2241,10 +2338,18 @@ __global__ void stage_pulses_kernel(const PulseDev *__restrict__ pulses, int n_p
     }
     // standard schedule: dt0, dt0 g, dt0 g^2, ... clipped to land on t1,
     // with exactly the lanes' arithmetic
-    double t = t0, h = pd.dt0;
+    double t = t0, h = pd.dt0, h_prev = 0.0, bound = err_floor;
     int n_std = 0;
     while (n_std < kMaxStd && t1 - t > kDblEps) {
-        if ((t + h) - t1 > kDblEps) h = t1 - t;
+        if ((t + h) - t1 > kDblEps) {
+            // the clipped last step: a lane takes it when its controller's step
+            // reaches t1, 0.9 err^(-1/8) h_prev > t1 - t, i.e. an error of the
+            // step before below (0.9 h_prev / (t1 - t))^8 (and below 0.5, where
+            // the controller starts to grow); 1e-6 off for the rounding
+            h = t1 - t;
+            const double q = 0.9 * h_prev / h, q2 = q * q, q4 = q2 * q2;
+            bound = fmax(err_floor, fmin(0.5, q4 * q4) * (1.0 - 1e-6));
+        }
         out[SCHED + 2 + n_std] = t;
         out[SCHED + 2 + kMaxStd + n_std] = h;
         for (int s = 0; s < 13; ++s) {
@@ -2254,9 +2359,11 @@ __global__ void stage_pulses_kernel(const PulseDev *__restrict__ pulses, int n_p
         }
         ++n_std;
         t += h;
+        h_prev = h;
         h *= grow_max;
     }
     out[SCHED] = (double)n_std;
+    out[SCHED + 1] = bound;
 }
 
 // j[p][i] = sum over the pulse's items of the partial rows, with Neumaier

@@ -141,7 +141,7 @@ template <int M, int D, int LAYOUT>
 void stage_one(const StageReq &s, unsigned blocks, int threads) {
     stage_pulses_kernel<M, D, LAYOUT><<<blocks, threads, 0, s.stream>>>(
         s.pulses, s.n_pulses, s.tgrid, s.interval_off, s.coef, s.total_intervals, s.grow_max,
-        s.gl30);
+        pow(5.0, -8.0), s.gl30);
 }
 
 template <int M, int D>
