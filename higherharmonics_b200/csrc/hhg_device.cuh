@@ -161,6 +161,12 @@ __host__ __device__ constexpr int slot_dyadic(int nf, int deg) { return slot_sch
 __host__ __device__ constexpr int slot_doubles_dyadic(int nf, int deg) {
     return slot_dyadic(nf, deg) + (((1 << kDyaLevels) - 1) * 13 * nf + 1) / 2 * 2;
 }
+// Magnus-4 layout (up to kMagnusTab substeps): after the header, per substep
+// the sum f(t_a) + f(t_b) and the difference f(t_b) - f(t_a) of the staged
+// functions at its two Gauss points, in the room of the interpolants and the
+// table.
+constexpr int kMagnusTab = kMaxStd * 13 / 2;
+constexpr double kGaussLo = 0.5 - 0.28867513459481288225;  // 1/2 - sqrt(3)/6
 // Value of staged function n outside the pulse window: A -> 0, cos -> 1, sin -> 0.
 template <int NF> __host__ __device__ constexpr double outside_value(int n) {
     return (NF > 1 && (n % 2) == 0) ? 1.0 : 0.0;
@@ -476,8 +482,14 @@ struct TableEval {
 // Models.  init() reads the k row and the pulse's scaled constants; rhs()
 // evaluates dS/dt in precision R from the pulse values f; vertex() is the
 // current contribution (weight excluded, FP64) from the sample record r =
-// [A(t_s), staged functions at t_s]; dvec() gives d with dS/dt = 2 d x S
-// (Magnus-4, FP64 only).
+// [A(t_s), staged functions at t_s].
+//
+// Magnus-4 (FP64 only; dS/dt = 2 d x S): omega() gives the rotation vector of
+// a step of size hs from the sum fp and the difference fm
+// of the staged functions at its Gauss points.  With p = d_a + d_b and m =
+// d_b - d_a, both linear in f, omega = hs (d_a + d_b) + sqrt(3)/3 hs^2 d_b x
+// d_a = P + M x P, P = hs p, M = sqrt(3)/6 hs m; each model leaves out its
+// vanishing components.
 //
 // The FP64 right-hand side is split by what each part depends on:
 // (PIFLUX3D_RELAX, whose result depends on its step sequence, keeps k = dS/dt
@@ -489,6 +501,7 @@ struct TableEval {
 //   eval(st, nd, S, k) k = h dS/dt at the state S.
 // ---------------------------------------------------------------------------
 template <int M, typename R> struct ModelState;
+constexpr double kMagnusCross = 0.28867513459481288225;  // sqrt(3)/6
 
 // gapped 2D Dirac, d = (v (kx - px A), v (ky - py A), mass); dS/dt = 2 d x S.
 // mp: [0] 2v, [1] 2 mass, [2] px, [3] py
@@ -532,10 +545,13 @@ template <typename R> struct ModelState<DIRAC2D, R> {
     __device__ __forceinline__ double vertex(const double *, const double *S) const {
         return px * S[0] + py * S[1];
     }
-    __device__ __forceinline__ void dvec(const double *f, double *d) const {
-        d[0] = 0.5 * N::lin(ax, bx, f[0]);
-        d[1] = 0.5 * N::lin(ay, by, f[0]);
-        d[2] = 0.5 * double(dz);
+    __device__ __forceinline__ void omega(double hs, const double *fp, const double *fm, double *w) const {
+        const double a = 0.5 * fp[0], m = -0.5 * kMagnusCross * hs * fm[0];
+        const double p0 = hs * (ax - bx * a), p1 = hs * (ay - by * a), p2 = hs * dz;
+        const double m0 = m * bx, m1 = m * by;
+        w[0] = p0 + m1 * p2;
+        w[1] = p1 - m0 * p2;
+        w[2] = p2 + (m0 * p1 - m1 * p0);
     }
 };
 
@@ -582,10 +598,13 @@ template <typename R> struct ModelState<PIFLUX3D, R> {
         // sin(k.z - A(t_i)) S_z (PiFlux.cpp:832-838)
         return (sz * r[1] - cz * r[2]) * S[2];
     }
-    __device__ __forceinline__ void dvec(const double *f, double *d) const {
-        d[0] = 0.5 * double(m0);
-        d[1] = 0.5 * double(m1);
-        d[2] = 0.5 * N::dot2(pcz, f[0], psz, f[1]);
+    __device__ __forceinline__ void omega(double hs, const double *fp, const double *fm, double *w) const {
+        const double h2 = 0.5 * hs;
+        const double p0 = hs * m0, p1 = hs * m1;
+        const double mz = kMagnusCross * h2 * (pcz * fm[0] + psz * fm[1]);
+        w[0] = p0 - mz * p1;
+        w[1] = p1 + mz * p0;
+        w[2] = h2 * (pcz * fp[0] + psz * fp[1]);
     }
 };
 
@@ -656,10 +675,11 @@ template <typename R, bool SYM> struct PiFlux2DState {
         // px sin(kx - px A) S_x + py sin(ky - py A) S_y
         return px * (sx * r[1] - cx * r[2]) * S[0] + py * (sy * r[1 + Y] - cy * r[2 + Y]) * S[1];
     }
-    __device__ __forceinline__ void dvec(const double *f, double *d) const {
-        d[0] = 0.5 * N::dot2(pcx, f[0], psx, f[1]);
-        d[1] = 0.5 * N::dot2(pcy, f[Y], psy, f[Y + 1]);
-        d[2] = 0.0;
+    __device__ __forceinline__ void omega(double hs, const double *fp, const double *fm, double *w) const {
+        const double a = 0.5 * pf * hs, b = kMagnusCross * a;
+        w[0] = a * (cx * fp[0] + sx * fp[1]);
+        w[1] = a * (cy * fp[Y] + sy * fp[Y + 1]);
+        w[2] = b * ((cx * fm[0] + sx * fm[1]) * w[1] - (cy * fm[Y] + sy * fm[Y + 1]) * w[0]);
     }
 };
 template <typename R> struct ModelState<PIFLUX2D, R> : PiFlux2DState<R, false> {};
@@ -786,19 +806,24 @@ template <typename R, bool X> struct HoneycombState {
         const double by = g1r * S[0] + g1i * S[1];
         return bx * px + by * py;
     }
-    __device__ __forceinline__ void dvec(const double *f, double *d) const {
-        // d = t (Re g', -Im g', mass) = 0.5 (pf Re g', -pf Im g', 2 mass)
-        double gre, gim;
-        if constexpr (X) {
-            gre = (c0 * f[0] + s0 * f[1]) + (c1 * f[2] + s1 * f[3]);
-            gim = (s0 * f[0] - c0 * f[1]) + (s1 * f[2] - c1 * f[3]);
-        } else {
-            gre = (c0 * f[0] + s0 * f[1]) + (c1 * f[2] + s1 * f[3]) + (c2 * f[Q2] + s2 * f[Q2 + 1]);
-            gim = (s0 * f[0] - c0 * f[1]) + (s1 * f[2] - c1 * f[3]) + (s2 * f[Q2] - c2 * f[Q2 + 1]);
+    // sum_j e^{i nn_j.k} e^{-i s_j A} for (linear combinations of) staged values f
+    __device__ __forceinline__ void bond_sum(const double *f, double &gre, double &gim) const {
+        gre = (c0 * f[0] + s0 * f[1]) + (c1 * f[2] + s1 * f[3]);
+        gim = (s0 * f[0] - c0 * f[1]) + (s1 * f[2] - c1 * f[3]);
+        if constexpr (!X) {
+            gre += c2 * f[Q2] + s2 * f[Q2 + 1];
+            gim += s2 * f[Q2] - c2 * f[Q2 + 1];
         }
-        d[0] = 0.5 * pf * gre;
-        d[1] = -0.5 * pf * gim;
-        d[2] = 0.5 * double(dm);
+    }
+    __device__ __forceinline__ void omega(double hs, const double *fp, const double *fm, double *w) const {
+        const double a = 0.5 * pf * hs, b = kMagnusCross * a;
+        double pr, pi, mr, mi;
+        bond_sum(fp, pr, pi);
+        bond_sum(fm, mr, mi);
+        const double p0 = a * pr, p1 = -a * pi, p2 = hs * dm, m0 = b * mr, m1 = -b * mi;
+        w[0] = p0 + m1 * p2;
+        w[1] = p1 - m0 * p2;
+        w[2] = p2 + (m0 * p1 - m1 * p0);
     }
 };
 template <typename R> struct ModelState<HONEYCOMB, R> : HoneycombState<R, false> {};
@@ -836,11 +861,11 @@ template <typename R> struct ModelState<DIRAC3D, R> {
         k[2] = -nd.mx * S[1];
     }
     __device__ __forceinline__ double vertex(const double *, const double *S) const { return S[2]; }
-    __device__ __forceinline__ void dvec(const double *f, double *d) const {
-        // G = [[0, mz, 0], [-mz, 0, mx], [0, -mx, 0]] = [g]_x, g = (-mx, 0, -mz) = 2 d
-        d[0] = -0.5 * N::mul(ax, f[0]);
-        d[1] = 0.0;
-        d[2] = -0.5 * N::lin(mk2, az, f[0]);
+    __device__ __forceinline__ void omega(double hs, const double *fp, const double *fm, double *w) const {
+        const double h2 = 0.5 * hs, m = kMagnusCross * h2 * fm[0];
+        w[0] = -h2 * (ax * fp[0]);
+        w[2] = h2 * (az * fp[0]) - hs * mk2;
+        w[1] = m * (az * w[0] + ax * w[2]);
     }
 };
 
@@ -1344,20 +1369,48 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Rodrigues rotation S <- exp([w]_x) S (series for theta < 1e-4).
-__device__ __forceinline__ void rotate(const double *w, double *S) {
-    const double th2 = w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
-    double sa, ca;
-    if (th2 < 1e-8) {
-        sa = 1.0 - th2 / 6.0 + th2 * th2 / 120.0;
-        ca = 0.5 - th2 / 24.0 + th2 * th2 / 720.0;
+// sin(theta) / theta and (1 - cos(theta)) / theta^2 as functions of x =
+// theta^2.  Up to x = 1 by their Taylor series (the first term left out is
+// below 1e-17 of the value): eight FMAs each, without a root, a quotient or a
+// range reduction; sampling intervals turn a trajectory by less than a radian
+// on all of the engine's workloads (0.3 to 0.8).
+// Larger angles take the library's functions, out of line.
+static __device__ __noinline__ double2 rotation_factors_large(double x) {
+    const double th = sqrt(x);
+    double sn, cs;
+    sincos(th, &sn, &cs);
+    return make_double2(sn / th, (1.0 - cs) / x);
+}
+__device__ __forceinline__ void rotation_factors(double x, double &sa, double &ca) {
+    if (x <= 1.0) {
+        double s = 1.0 / 355687428096000.0, c = 1.0 / 6402373705728000.0;  // 1/17!, 1/18!
+        s = fma(s, x, -1.0 / 1307674368000.0);
+        c = fma(c, x, -1.0 / 20922789888000.0);
+        s = fma(s, x, 1.0 / 6227020800.0);
+        c = fma(c, x, 1.0 / 87178291200.0);
+        s = fma(s, x, -1.0 / 39916800.0);
+        c = fma(c, x, -1.0 / 479001600.0);
+        s = fma(s, x, 1.0 / 362880.0);
+        c = fma(c, x, 1.0 / 3628800.0);
+        s = fma(s, x, -1.0 / 5040.0);
+        c = fma(c, x, -1.0 / 40320.0);
+        s = fma(s, x, 1.0 / 120.0);
+        c = fma(c, x, 1.0 / 720.0);
+        s = fma(s, x, -1.0 / 6.0);
+        c = fma(c, x, -1.0 / 24.0);
+        sa = fma(s, x, 1.0);
+        ca = fma(c, x, 0.5);
     } else {
-        const double th = sqrt(th2);
-        double s, c;
-        sincos(th, &s, &c);
-        sa = s / th;
-        ca = (1.0 - c) / th2;
+        const double2 f = rotation_factors_large(x);
+        sa = f.x;
+        ca = f.y;
     }
+}
+
+// Rodrigues rotation S <- exp([w]_x) S.
+__device__ __forceinline__ void rotate(const double *w, double *S) {
+    double sa, ca;
+    rotation_factors(w[0] * w[0] + w[1] * w[1] + w[2] * w[2], sa, ca);
     const double wx0 = w[1] * S[2] - w[2] * S[1];
     const double wx1 = w[2] * S[0] - w[0] * S[2];
     const double wx2 = w[0] * S[1] - w[1] * S[0];
@@ -1618,6 +1671,17 @@ __device__ __forceinline__ void lane_controller(const KParams &P, const ModelSta
     if (alive) attempts_out += attempts;
 }
 
+// N values (N even, 16-byte aligned) with 16-byte loads through the read-only path.
+template <int N> __device__ __forceinline__ void load_even(const double *src, double *v) {
+    static_assert(N % 2 == 0, "pairs");
+#pragma unroll
+    for (int n = 0; n < N; n += 2) {
+        const double2 w = __ldg(reinterpret_cast<const double2 *>(src + n));
+        v[n] = w.x;
+        v[n + 1] = w.y;
+    }
+}
+
 __device__ __forceinline__ void copy16_async(void *smem, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
                  :
@@ -1629,7 +1693,13 @@ __device__ __forceinline__ void copy16_async(void *smem, const void *gmem) {
 // Persistent, work-stealing integration + BZ-sum kernel.
 // STEPPER 0: controlled RKF78; STEPPER 1: Magnus-4 (two-point Gauss),
 //   magnus_substeps steps per interval: omega = h (d1 + d2) + (sqrt3/3) h^2
-//   (d2 x d1), S <- exp([omega]_x) S.
+//   (d2 x d1), S <- exp([omega]_x) S, from the staged sums and differences
+//   (up to kMagnusTab substeps; STEPPER 3: more, from the interpolants).  The
+//   Gauss-point values, formerly two interpolants per staged function
+//   evaluated by every lane, and the rotation (a root, a sine and cosine, two
+//   quotients) were two thirds of the 199 FP64 instructions of an interval
+//   (honeycomb):
+//   512 x 512, 6144 intervals, 42.7 -> 15.2 ms a spectrum, 89 FP64 instructions.
 // PROPOSER 0: the reference's per-lane controller, every interval restarting
 //   at dt0 = measure_every / n_subdivisions;
 // PROPOSER 1: per-lane controller, an interval starts from the controller's
@@ -1844,15 +1914,17 @@ bz_integrate_kernel(const KParams P) {
     // is read from global memory
     // the relaxation models on the reference schedule run free lanes (above)
     constexpr bool kFree = Traits<M>::kRelax && PROPOSER == 0 && STEPPER == 0 && OUT == 0;
-    constexpr int COPY = kFree ? 2 : (PROPOSER == 0) ? SLOT : SCHED;
+    // (Magnus-4: the header and the first substep's sums and differences)
+    constexpr int COPY = kFree ? 2 : STEPPER == 1 ? slot_poly(NF) + 2 * NF : (PROPOSER == 0) ? SLOT : SCHED;
     constexpr int NTAB = kMaxStd * 13 * NF;
     using V = typename Num<R>::V;
-    // FP64 RKF78: interval records are copied one interval ahead (cp.async) into
-    // two buffers, and samples are summed eight at a time (put_sample)
-    constexpr bool kFetch = STEPPER == 0 && !kNarrow && !kFree;
+    // FP64 RKF78 and Magnus-4: interval records are copied one interval ahead
+    // (cp.async) into two buffers, and samples are summed eight at a time
+    // (put_sample)
+    constexpr bool kFetch = (STEPPER == 0 && !kNarrow && !kFree) || STEPPER == 1;
     __shared__ __align__(16) double stage_raw[kWarpsPerBlock][kFetch ? 2 : 1][COPY];
     __shared__ double free_ring[kWarpsPerBlock][kFree ? kFreeWindow * 32 : 1];
-    constexpr bool kRingSum = STEPPER == 0 && !kNarrow && !kFree && OUT == 0;
+    constexpr bool kRingSum = kFetch && OUT == 0;
     __shared__ double ring[kWarpsPerBlock][kRingSum ? kRing * kRingRow : 1];
     __shared__ __align__(16) V stage_tab[kWarpsPerBlock][kNarrow && PROPOSER == 0 ? NTAB : 1];
     // learned proposer: per-warp input tiles in dynamic shared memory
@@ -1902,17 +1974,6 @@ bz_integrate_kernel(const KParams P) {
             double held2 = 0.0; // ... and of its second channel (OUT 1)
             double kc[4];       // momentum cosines (OUT 1-3)
             if constexpr (OUT >= 1 && OUT <= 3) piflux_cosines(row, kc);
-            // Magnus-4 with one step per interval: the next interval's pulse
-            // values at its two Gauss points, evaluated one interval ahead
-            // (off the rotation's dependency chain)
-            constexpr double kGa = 0.5 - 0.28867513459481288225;
-            double ga_next[STEPPER == 1 ? NF : 1], gb_next[STEPPER == 1 ? NF : 1];
-            if constexpr (STEPPER == 1) {
-                const double h0 = coef[1] - coef[0];
-                const PolyEval<NF, D, double> pe{coef, tb, te, &pd};
-                pe(0, coef[0] + kGa * h0, ga_next);
-                pe(0, coef[0] + (1.0 - kGa) * h0, gb_next);
-            }
             // closed-form Magnus step: the next interval's moments are loaded
             // while the current step computes (registers, off the step's chain)
             double mom_next[4] = {0.0, 0.0, 0.0, 0.0};
@@ -1942,10 +2003,9 @@ bz_integrate_kernel(const KParams P) {
             for (int i = 0; i <= N; ++i) {
                 const double *rec = pd.s0rec;
                 if (i > 0) {
-                    // interval i-1 in this warp's shared slot (the Magnus
-                    // steppers read their interpolants or moments and the
-                    // record straight from the staging table: warp broadcasts
-                    // of a few values per interval)
+                    // interval i-1 in this warp's shared slot (the closed-form
+                    // Magnus step reads its moments and the record straight from
+                    // the staging table: warp broadcasts of a few values)
                     const double *gslot = coef + (size_t)(i - 1) * SLOT;
                     if constexpr (kFetch) {
                         slot = stage_raw[wib][(i - 1) & 1];
@@ -1976,54 +2036,43 @@ bz_integrate_kernel(const KParams P) {
                         }
                         __syncwarp();
                     }
-                    const double *cur = STEPPER != 0 ? gslot : slot;
+                    const double *cur = kFetch || STEPPER == 0 ? slot : gslot;
                     rec = cur + 4;
                     const double t0 = cur[0], t1 = cur[1];
                     const PolyEval<NF, D, R, kPair> poly{slot, tb, te, &pd};
                     if constexpr (STEPPER == 1) {
-                        if (P.magnus_substeps == 1) {
-                            double f1[NF], f2[NF];
+                        const int ns = P.magnus_substeps;
+                        const double hs = ns == 1 ? t1 - t0 : (t1 - t0) / ns;
+                        if (!dead) {
+                            double f[2 * NF];
 #pragma unroll
-                            for (int n = 0; n < NF; ++n) {
-                                f1[n] = ga_next[n];
-                                f2[n] = gb_next[n];
-                            }
-                            if (i < N) {
-                                const double *gn = gslot + SLOT;
-                                const double hn = gn[1] - gn[0];
-                                const PolyEval<NF, D, double> pe{gn, tb, te, &pd};
-                                pe(0, gn[0] + kGa * hn, ga_next);
-                                pe(0, gn[0] + (1.0 - kGa) * hn, gb_next);
-                            }
-                            if (!dead) {
-                                const double hs = t1 - t0;
-                                const double q3 = 0.57735026918962576451 * hs * hs;
-                                double d1[3], d2[3], wv[3];
-                                ms.dvec(f1, d1);
-                                ms.dvec(f2, d2);
-                                wv[0] = hs * (d1[0] + d2[0]) + q3 * (d2[1] * d1[2] - d2[2] * d1[1]);
-                                wv[1] = hs * (d1[1] + d2[1]) + q3 * (d2[2] * d1[0] - d2[0] * d1[2]);
-                                wv[2] = hs * (d1[2] + d2[2]) + q3 * (d2[0] * d1[1] - d2[1] * d1[0]);
+                            for (int n = 0; n < 2 * NF; ++n) f[n] = slot[slot_poly(NF) + n];
+                            for (int s = 0;;) {
+                                double wv[3];
+                                ms.omega(hs, f, f + NF, wv);
                                 rotate(wv, S);
-                                ++my_attempts;
+                                if (++s == ns) break;
+                                load_even<2 * NF>(gslot + slot_poly(NF) + s * (2 * NF), f);
                             }
-                        } else if (!dead) {
+                            my_attempts += ns;
+                        }
+                    } else if constexpr (STEPPER == 3) {
+                        if (!dead) {
                             const int ns = P.magnus_substeps;
                             const double hs = (t1 - t0) / ns;
-                            const double g = 0.5 - 0.28867513459481288225;
-                            const double q3 = 0.57735026918962576451 * hs * hs;
                             for (int s = 0; s < ns; ++s) {
                                 const double ts = t0 + s * hs;
-                                double f[NF], d1[3], d2[3];
+                                double f1[NF], f2[NF], wv[3];
                                 const PolyEval<NF, D, double> pd64{cur, tb, te, &pd};
-                                pd64(0, ts + g * hs, f);
-                                ms.dvec(f, d1);
-                                pd64(0, ts + (1.0 - g) * hs, f);
-                                ms.dvec(f, d2);
-                                double wv[3];
-                                wv[0] = hs * (d1[0] + d2[0]) + q3 * (d2[1] * d1[2] - d2[2] * d1[1]);
-                                wv[1] = hs * (d1[1] + d2[1]) + q3 * (d2[2] * d1[0] - d2[0] * d1[2]);
-                                wv[2] = hs * (d1[2] + d2[2]) + q3 * (d2[0] * d1[1] - d2[1] * d1[0]);
+                                pd64(0, ts + kGaussLo * hs, f1);
+                                pd64(0, ts + (1.0 - kGaussLo) * hs, f2);
+#pragma unroll
+                                for (int n = 0; n < NF; ++n) {
+                                    const double d = f2[n] - f1[n];
+                                    f1[n] += f2[n];
+                                    f2[n] = d;
+                                }
+                                ms.omega(hs, f1, f2, wv);
                                 rotate(wv, S);
                             }
                             my_attempts += ns;
@@ -2221,7 +2270,7 @@ __global__ void stage_pulses_kernel(const PulseDev *__restrict__ pulses, int n_p
                                     double grow_max, double err_floor,
                                     const double *__restrict__ gl30) {
     constexpr int NF = Traits<M>::NF;
-    constexpr int SLOT = (LAYOUT == 0 || LAYOUT == 3) ? slot_doubles(NF, D) : slot_doubles_dyadic(NF, D);
+    constexpr int SLOT = (LAYOUT == 1 || LAYOUT == 2) ? slot_doubles_dyadic(NF, D) : slot_doubles(NF, D);
     constexpr int HDR = slot_header(NF);
     constexpr int SCHED = slot_sched(NF, D);
     constexpr int TAB = slot_table(NF, D);
@@ -2364,6 +2413,49 @@ __global__ void stage_pulses_kernel(const PulseDev *__restrict__ pulses, int n_p
     }
     out[SCHED] = (double)n_std;
     out[SCHED + 1] = bound;
+}
+
+// Staging for Magnus-4 with up to kMagnusTab substeps: the header (as above)
+// and the sums and differences at the Gauss points, no interpolants.
+template <int M, int D>
+__global__ void stage_magnus_kernel(const PulseDev *__restrict__ pulses, int n_pulses,
+                                    const double *__restrict__ tgrid,
+                                    const long long *__restrict__ interval_off,
+                                    double *__restrict__ coef, long long total_intervals,
+                                    int substeps) {
+    constexpr int NF = Traits<M>::NF;
+    const long long gid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (gid >= total_intervals) return;
+    int lo = 0, hi = n_pulses;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (interval_off[mid] <= gid) lo = mid; else hi = mid;
+    }
+    const int i = (int)(gid - interval_off[lo]);
+    const PulseDev pd = pulses[lo];
+    const double *tg = tgrid + interval_off[lo] + lo + i;
+    const double t0 = tg[0], t1 = tg[1];
+    double *out = coef + pd.coef_off + (long long)i * slot_doubles(NF, D);
+    const double As = laser_exact(pd, (i + 1) * pd.measure_every + pd.window_begin);
+    double v[NF], u[NF];
+    staged_values<M>(pd, As, v);
+    out[0] = t0;
+    out[1] = t1;
+    out[2] = 0.5 * (t0 + t1);
+    out[3] = 1.0 / (0.5 * (t1 - t0));
+    out[4] = As;
+    for (int n = 0; n < NF; ++n) out[5 + n] = v[n];
+    const double hs = (t1 - t0) / substeps;
+    double *o = out + slot_poly(NF);
+    for (int q = 0; q < substeps; ++q, o += 2 * NF) {
+        const double ts = t0 + q * hs;
+        staged_values<M>(pd, laser_exact(pd, ts + kGaussLo * hs), v);
+        staged_values<M>(pd, laser_exact(pd, ts + (1.0 - kGaussLo) * hs), u);
+        for (int n = 0; n < NF; ++n) {
+            o[n] = v[n] + u[n];
+            o[NF + n] = u[n] - v[n];
+        }
+    }
 }
 
 // j[p][i] = sum over the pulse's items of the partial rows, with Neumaier

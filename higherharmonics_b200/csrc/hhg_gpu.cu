@@ -1225,7 +1225,9 @@ static hhg_status plan_create_impl(hhg_ctx *ctx, const hhg_system_desc *sys,
     }
     pl->degree = exact ? 0 : degree;
     degree = pl->degree;
-    const bool dyadic = o.proposer == HHG_PROPOSER_LOCKSTEP || o.proposer == HHG_PROPOSER_LEARNED;
+    // (the Magnus steppers have no step proposer and read the standard slots)
+    const bool dyadic = o.stepper == HHG_STEPPER_RKF78 &&
+                        (o.proposer == HHG_PROPOSER_LOCKSTEP || o.proposer == HHG_PROPOSER_LEARNED);
     const int slot = dyadic ? hhg::slot_doubles_dyadic(nf, degree) : hhg::slot_doubles(nf, degree);
 
     // work decomposition
@@ -1404,6 +1406,10 @@ static hhg_status plan_create_impl(hhg_ctx *ctx, const hhg_system_desc *sys,
                      pl->n_intervals, degree, 9.0 / 10.0 * pow(pow(5.0, -8.0), -1.0 / 8), s};
     sr.layout = dyadic ? (o.precision == HHG_PREC_MIXED ? 2 : 1) : (magnus_moments ? 3 : 0);
     if (magnus_moments) sr.gl30 = pl->d_coef + gl_off;
+    if (o.stepper == HHG_STEPPER_MAGNUS4 && o.magnus_substeps <= hhg::kMagnusTab) {
+        sr.layout = 4;
+        sr.substeps = o.magnus_substeps;
+    }
     if ((st = stage_variant(pl, sr)) != HHG_OK) {
         hhg_plan_destroy(pl);
         return st;
@@ -1415,6 +1421,7 @@ static hhg_status plan_create_impl(hhg_ctx *ctx, const hhg_system_desc *sys,
     lr.precision = o.precision;
     lr.stepper = o.stepper;
     lr.proposer = kernel_proposer(o.proposer);
+    lr.kp.magnus_substeps = o.magnus_substeps;
     lr.grid = 0;
     lr.occupancy_out = &occ;
     if ((st = launch_variant(pl, lr)) != HHG_OK) {

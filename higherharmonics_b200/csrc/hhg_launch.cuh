@@ -31,7 +31,9 @@ struct StageReq {
     int degree;
     double grow_max;
     cudaStream_t stream;
-    int layout = 0;  // 0 standard schedule, 1 dyadic FP64, 2 dyadic float pairs, 3 Dirac Magnus moments
+    int layout = 0;  // 0 standard schedule, 1 dyadic FP64, 2 dyadic float pairs, 3 Dirac Magnus moments,
+                     // 4 Magnus-4 sums and differences
+    int substeps = 1;  // layout 4: Magnus-4 substeps per interval, <= kMagnusTab
     const double *gl30 = nullptr;  // layout 3: 30 nodes on [0, 1], then 30 weights (device)
 };
 
@@ -96,7 +98,9 @@ cudaError_t launch_deg(const LaunchReq &r) {
             if constexpr (M == DIRAC3D) return launch_one<M, D, double, 2, 0>(r);
             else return cudaErrorNotSupported;
         }
-        if (r.stepper == 1) return launch_one<M, D, double, 1, 0>(r);
+        if (r.stepper == 1)
+            return r.kp.magnus_substeps <= kMagnusTab ? launch_one<M, D, double, 1, 0>(r)
+                                                      : launch_one<M, D, double, 3, 0>(r);
         if (r.precision == 0) {
             switch (r.proposer) {
             case 0: return launch_one<M, D, double, 0, 0>(r);
@@ -149,14 +153,19 @@ void stage_deg(const StageReq &s, unsigned blocks, int threads) {
     if (s.layout == 0) stage_one<M, D, 0>(s, blocks, threads);
     else if (s.layout == 1) stage_one<M, D, 1>(s, blocks, threads);
     else if (s.layout == 2) stage_one<M, D, 2>(s, blocks, threads);
-    else if constexpr (M == DIRAC3D) stage_one<M, D, 3>(s, blocks, threads);
+    else if (s.layout == 4) {
+        if constexpr (!Traits<M>::kRelax)
+            stage_magnus_kernel<M, D><<<blocks, threads, 0, s.stream>>>(
+                s.pulses, s.n_pulses, s.tgrid, s.interval_off, s.coef, s.total_intervals, s.substeps);
+    } else if constexpr (M == DIRAC3D) stage_one<M, D, 3>(s, blocks, threads);
 }
 
 template <int M>
 cudaError_t stage_model(const StageReq &s) {
     const int threads = 128;
     const long long blocks = (s.total_intervals + threads - 1) / threads;
-    if (s.layout < 0 || s.layout > 3 || (s.layout == 3 && (M != DIRAC3D || !s.gl30)))
+    if (s.layout < 0 || s.layout > 4 || (s.layout == 3 && (M != DIRAC3D || !s.gl30)) ||
+        (s.layout == 4 && (Traits<M>::kRelax || s.substeps < 1 || s.substeps > kMagnusTab)))
         return cudaErrorInvalidValue;
     if (s.degree == 0) {
         if (s.layout != 0) return cudaErrorNotSupported;

@@ -310,6 +310,10 @@ extern "C" hhg_status hhg_gpu_current_density_noalloc(const hhg_system_desc *sys
 
     const double grow_max = 9.0 / 10.0 * pow(pow(5.0, -8.0), -1.0 / 8);
     hhg::StageReq sr{d_pulse, 1, d_tgrid, d_ioff, d_coef, (long long)N, prep.degree, grow_max, s};
+    if (o.stepper == HHG_STEPPER_MAGNUS4 && o.magnus_substeps <= hhg::kMagnusTab) {
+        sr.layout = 4;
+        sr.substeps = o.magnus_substeps;
+    }
     if ((e = stage_model(prep.model, sr)) != cudaSuccess) return fail(e);
 
     hhg::LaunchReq lr{};
