@@ -519,11 +519,13 @@ template <typename R> struct ModelState<DIRAC2D, R> {
         px = p.mp[2];
         py = p.mp[3];
     }
-    __device__ __forceinline__ void rhs(const typename N::V *f, const R *S, R *dS) const {
-        const R d0 = R(N::lin(ax, bx, f[0])), d1 = R(N::lin(ay, by, f[0]));
-        dS[0] = d1 * S[2] - dz * S[1];
-        dS[1] = dz * S[0] - d0 * S[2];
-        dS[2] = d0 * S[1] - d1 * S[0];
+    __device__ __forceinline__ float2 node32(const float2 *f) const {
+        return make_float2(N::lin(ax, bx, f[0]), N::lin(ay, by, f[0]));
+    }
+    __device__ __forceinline__ void eval32(float2 d, const float *S, float *dS) const {
+        dS[0] = d.y * S[2] - dz * S[1];
+        dS[1] = dz * S[0] - d.x * S[2];
+        dS[2] = d.x * S[1] - d.y * S[0];
     }
     struct Step {
         double ax, ay, bx, by, dz;
@@ -570,10 +572,12 @@ template <typename R> struct ModelState<PIFLUX3D, R> {
         pcz = N::mk(pf * cz);
         psz = N::mk(pf * sz);
     }
-    __device__ __forceinline__ void rhs(const typename N::V *f, const R *S, R *dS) const {
-        const R m2 = R(N::dot2(pcz, f[0], psz, f[1]));
-        dS[0] = m1 * S[2] - m2 * S[1];
-        dS[1] = m2 * S[0] - m0 * S[2];
+    __device__ __forceinline__ float2 node32(const float2 *f) const {
+        return make_float2(N::dot2(pcz, f[0], psz, f[1]), 0.f);
+    }
+    __device__ __forceinline__ void eval32(float2 m2, const float *S, float *dS) const {
+        dS[0] = m1 * S[2] - m2.x * S[1];
+        dS[1] = m2.x * S[0] - m0 * S[2];
         dS[2] = m0 * S[1] - m1 * S[0];
     }
     struct Step {
@@ -654,8 +658,7 @@ template <typename R, bool SYM> struct PiFlux2DState {
     // FP32 on packed pairs: (m0, m1) = Num<float>::dot2 of both projections in
     // one set of paired FMAs, then dS = (m1 Sz, -m0 Sz, m0 Sy - m1 Sx)
     // (the non-symmetric model's staged values arrive in the paired layout)
-    __device__ __forceinline__ void rhs2(const float2 *f, float2 s_xy, float s_z, float2 &d_xy,
-                                         float &d_z) const {
+    __device__ __forceinline__ float2 node32(const float2 *f) const {
         float2 bhi, blo, dhi, dlo;
         if constexpr (SYM) {
             bhi = make_float2(f[0].x, f[0].x), blo = make_float2(f[0].y, f[0].y);
@@ -667,7 +670,9 @@ template <typename R, bool SYM> struct PiFlux2DState {
         lo = __ffma2_rn(pc_lo, bhi, lo);
         lo = __ffma2_rn(ps_hi, dlo, lo);
         lo = __ffma2_rn(ps_lo, dhi, lo);
-        const float2 m = __ffma2_rn(pc_hi, bhi, __ffma2_rn(ps_hi, dhi, lo));
+        return __ffma2_rn(pc_hi, bhi, __ffma2_rn(ps_hi, dhi, lo));
+    }
+    __device__ __forceinline__ void eval2(float2 m, float2 s_xy, float s_z, float2 &d_xy, float &d_z) const {
         d_xy = __fmul2_rn(make_float2(m.y, -m.x), make_float2(s_z, s_z));
         d_z = fmaf(m.x, s_xy.y, -(m.y * s_xy.x));
     }
@@ -765,24 +770,30 @@ template <typename R, bool X> struct HoneycombState {
         k[1] = st.dm * S[0] - S[2] * nd.gr;
         k[2] = S[0] * nd.gi + S[1] * nd.gr;
     }
-    __device__ __forceinline__ void rhs(const typename N::V *f, const R *S, R *dS) const {
-        R gr, gi;
-        gamma(f, gr, gi);
-        dS[0] = -(S[2] * gi) - dm * S[1];
-        dS[1] = -(S[2] * gr) + dm * S[0];
-        dS[2] = S[0] * gi + S[1] * gr;
-    }
     // FP32, field along x, staged values in the leading-pairs-first layout
     // (f[0] = hi cos of both projections, f[1] = hi sin): the two bond
     // groups' products of the leading parts (no compensation: see Num) sit in
     // the two halves of paired FMAs, summed at the end:
     // pf Re g' = PC.FC + PS.FS, pf Im g' = PS.FC - PC.FS.
-    __device__ __forceinline__ void rhs2(const float2 *f, float2 s_xy, float s_z, float2 &d_xy,
-                                         float &d_z) const {
+    __device__ __forceinline__ float2 node32(const float2 *f) const {
+        if constexpr (X) {
+            const float2 re = __ffma2_rn(pc_hi, f[0], __fmul2_rn(ps_hi, f[1]));
+            const float2 im = __ffma2_rn(ps_hi, f[0], __fmul2_rn(mc_hi, f[1]));
+            return make_float2(re.x + re.y, im.x + im.y);
+        } else {
+            R gr, gi;
+            gamma(f, gr, gi);
+            return make_float2(gr, gi);
+        }
+    }
+    __device__ __forceinline__ void eval32(float2 g, const float *S, float *dS) const {
+        dS[0] = -(S[2] * g.y) - dm * S[1];
+        dS[1] = -(S[2] * g.x) + dm * S[0];
+        dS[2] = S[0] * g.y + S[1] * g.x;
+    }
+    __device__ __forceinline__ void eval2(float2 g, float2 s_xy, float s_z, float2 &d_xy, float &d_z) const {
         static_assert(X, "paired right-hand side: field along x");
-        const float2 re = __ffma2_rn(pc_hi, f[0], __fmul2_rn(ps_hi, f[1]));
-        const float2 im = __ffma2_rn(ps_hi, f[0], __fmul2_rn(mc_hi, f[1]));
-        const float gr = re.x + re.y, gi = im.x + im.y;
+        const float gr = g.x, gi = g.y;
         const float dmf = float(dm);
         d_xy = make_float2(fmaf(-s_z, gi, -(dmf * s_xy.y)), fmaf(-s_z, gr, dmf * s_xy.x));
         d_z = fmaf(s_xy.x, gi, s_xy.y * gr);
@@ -838,12 +849,13 @@ template <typename R> struct ModelState<DIRAC3D, R> {
         az = N::mk(2.0 * row[0] / row[2]);
         mk2 = N::mk(2.0 * row[2]);
     }
-    __device__ __forceinline__ void rhs(const typename N::V *f, const R *S, R *dS) const {
-        const R mx = R(N::mul(ax, f[0]));
-        const R mz = R(N::lin(mk2, az, f[0]));
-        dS[0] = mz * S[1];
-        dS[1] = mx * S[2] - S[0] * mz;
-        dS[2] = -mx * S[1];
+    __device__ __forceinline__ float2 node32(const float2 *f) const {
+        return make_float2(N::mul(ax, f[0]), N::lin(mk2, az, f[0]));
+    }
+    __device__ __forceinline__ void eval32(float2 m, const float *S, float *dS) const {
+        dS[0] = m.y * S[1];
+        dS[1] = m.x * S[2] - S[0] * m.y;
+        dS[2] = -m.x * S[1];
     }
     struct Step {
         double ax, az, mk2;
@@ -1087,15 +1099,18 @@ __device__ __forceinline__ void piflux_cosines(const double *row, double *c) {
 // the stage arithmetic counts directly.  Same tableau, same grouping of the
 // sums as rkf78_attempt.
 // ---------------------------------------------------------------------------
-template <int M, class V>
-__device__ __forceinline__ void rhs_packed(const ModelState<M, float> &ms, const V *f, float2 s_xy,
-                                           float s_z, float2 &d_xy, float &d_z) {
+// The right-hand side is split as the FP64 one: node32() holds the two numbers
+// that depend on the momentum and the time, once per node of the tableau
+// (stages 7, 11 and 12 sit on the nodes of stages 3, 0 and 10).
+template <int M>
+__device__ __forceinline__ void eval_packed(const ModelState<M, float> &ms, float2 nd, float2 s_xy,
+                                            float s_z, float2 &d_xy, float &d_z) {
     if constexpr (Traits<M>::kPacked) {
-        ms.rhs2(f, s_xy, s_z, d_xy, d_z);
+        ms.eval2(nd, s_xy, s_z, d_xy, d_z);
     } else {
         const float S[3] = {s_xy.x, s_xy.y, s_z};
         float d[3];
-        ms.rhs(f, S, d);
+        ms.eval32(nd, S, d);
         d_xy = make_float2(d[0], d[1]);
         d_z = d[2];
     }
@@ -1118,29 +1133,22 @@ __device__ __forceinline__ void rkf78_attempt_packed(const ModelState<M, float> 
     const float hr = float(h);
     const float2 h2 = make_float2(hr, hr);
     ev(0, t, f);
-    rhs_packed(ms, f, x2, xz, k2[0], kz[0]);
-    typename Num<float>::V f0[Eval::kReuse ? NF : 1], f3[Eval::kReuse ? NF : 1],
-        f10[Eval::kReuse ? NF : 1];
-    if constexpr (Eval::kReuse) {
-#pragma unroll
-        for (int n = 0; n < NF; ++n) f0[n] = f[n];
-    }
+    const float2 n0 = ms.node32(f);
+    float2 n3 = n0, n10 = n0;
+    eval_packed(ms, n0, x2, xz, k2[0], kz[0]);
 #define HHG_PSTAGE(s, SUM2, SUMZ)                                                   \
     {                                                                               \
         const float2 xt2 = __ffma2_rn(h2, (SUM2), x2);                              \
         const float xtz = xz + hr * (SUMZ);                                         \
-        if constexpr (Eval::kReuse && (s == 7 || s == 11 || s == 12)) {             \
-            _Pragma("unroll") for (int n = 0; n < NF; ++n)                          \
-                f[n] = (s == 7) ? f3[n] : (s == 11) ? f0[n] : f10[n];               \
+        if constexpr (s == 7 || s == 11 || s == 12) {                               \
+            eval_packed(ms, s == 7 ? n3 : s == 11 ? n0 : n10, xt2, xtz, k2[s], kz[s]); \
         } else {                                                                    \
             ev(s, t + rk_c(s) * h, f);                                              \
+            const float2 nd = ms.node32(f);                                         \
+            if constexpr (s == 3) n3 = nd;                                          \
+            if constexpr (s == 10) n10 = nd;                                        \
+            eval_packed(ms, nd, xt2, xtz, k2[s], kz[s]);                            \
         }                                                                           \
-        if constexpr (Eval::kReuse && (s == 3 || s == 10)) {                        \
-            _Pragma("unroll") for (int n = 0; n < NF; ++n) {                        \
-                if (s == 3) f3[n] = f[n]; else f10[n] = f[n];                       \
-            }                                                                       \
-        }                                                                           \
-        rhs_packed(ms, f, xt2, xtz, k2[s], kz[s]);                               \
     }
 #define Z(c, j) (float(c) * kz[j])
     HHG_PSTAGE(1, pmul(2.0 / 27.0, k2[0]), Z(2.0 / 27.0, 0))
@@ -1315,7 +1323,7 @@ __device__ __forceinline__ void rkf78_attempt(const ModelState<M, R> &ms, const 
         const auto st = ms.step(h);
         ev(0, t, f);
         const Node n0 = ms.node(st, f);
-        Node n3, n10;
+        Node n3 = n0, n10 = n0;
         ms.eval(st, n0, x, k[0]);
 #define HHG_STAGE(s, CHAIN)                                                         \
     {                                                                               \
@@ -1878,11 +1886,12 @@ constexpr int kCoarsenDivMixed = 64;
 // worth more than a fourth warp: 7 -> 5 CTAs, honeycomb 512 x 512 8.08 ->
 // 7.35 ms (256 intervals), pi-flux 256 x 256 3.47 -> 3.37 ms (512 intervals).
 // The lattice models' relaxation: 4 (255 registers; at 168 the stage values
-// spill, 1.7x slower).
+// spill, 1.7x slower).  Mixed precision: 7 (128 registers), pi-flux 5 (1.62 ->
+// 1.54 ms at 256 x 256 and 1024 intervals; honeycomb and Dirac lose 1-9 %).
 __host__ __device__ constexpr int min_blocks(int model, bool fp64, int stepper) {
-    return fp64 && stepper == 0 && model != PIFLUX3D_RELAX && model != HONEYCOMB_RELAX ? 5
-           : model == PIFLUX3D_RELAX || model == HONEYCOMB_RELAX                       ? 4
-                                                                                       : kMinBlocksPerSM;
+    return model == PIFLUX3D_RELAX || model == HONEYCOMB_RELAX ? 4
+           : fp64 ? (stepper == 0 ? 5 : kMinBlocksPerSM)
+           : model == PIFLUX2D || model == PIFLUX2D_SYM ? 5 : kMinBlocksPerSM;
 }
 
 // OUT 0: the Brillouin-zone sum of the current (one partial row per item);
@@ -1915,13 +1924,18 @@ bz_integrate_kernel(const KParams P) {
     // the relaxation models on the reference schedule run free lanes (above)
     constexpr bool kFree = Traits<M>::kRelax && PROPOSER == 0 && STEPPER == 0 && OUT == 0;
     // (Magnus-4: the header and the first substep's sums and differences)
-    constexpr int COPY = kFree ? 2 : STEPPER == 1 ? slot_poly(NF) + 2 * NF : (PROPOSER == 0) ? SLOT : SCHED;
+    // (dyadic steppers: up to the end of the level-0 stage table)
+    constexpr int COPY = kFree           ? 2
+                         : STEPPER == 1  ? slot_poly(NF) + 2 * NF
+                         : kDyadic       ? DYA + ((13 * NF + 1) & ~1)
+                         : PROPOSER == 0 ? SLOT
+                                         : SCHED;
     constexpr int NTAB = kMaxStd * 13 * NF;
     using V = typename Num<R>::V;
     // FP64 RKF78 and Magnus-4: interval records are copied one interval ahead
     // (cp.async) into two buffers, and samples are summed eight at a time
     // (put_sample)
-    constexpr bool kFetch = (STEPPER == 0 && !kNarrow && !kFree) || STEPPER == 1;
+    constexpr bool kFetch = (STEPPER == 0 && (!kNarrow || kDyadic) && !kFree) || STEPPER == 1;
     __shared__ __align__(16) double stage_raw[kWarpsPerBlock][kFetch ? 2 : 1][COPY];
     __shared__ double free_ring[kWarpsPerBlock][kFree ? kFreeWindow * 32 : 1];
     constexpr bool kRingSum = kFetch && OUT == 0;
@@ -1982,10 +1996,16 @@ bz_integrate_kernel(const KParams P) {
                 for (int c = 0; c < 4; ++c) mom_next[c] = __ldg(coef + TAB + c);
             }
 
+            // (one running pointer per 32 pieces of 16 bytes)
+            constexpr int kPieces = (COPY / 2 + 31) / 32;
+            const double *fsrc = coef + 2 * lane;
             auto fetch = [&](int interval) {
-                const double *src = coef + (size_t)interval * SLOT;
-                double *dst = stage_raw[wib][interval & (kFetch ? 1 : 0)];
-                for (int c = lane; c < COPY / 2; c += 32) copy16_async(dst + 2 * c, src + 2 * c);
+                double *dst = stage_raw[wib][interval & (kFetch ? 1 : 0)] + 2 * lane;
+#pragma unroll
+                for (int q = 0; q < kPieces; ++q)
+                    if (32 * (q + 1) <= COPY / 2 || lane < COPY / 2 - 32 * q)
+                        copy16_async(dst + 64 * q, fsrc + 64 * q);
+                fsrc += SLOT;
                 asm volatile("cp.async.commit_group;" ::: "memory");
             };
             if constexpr (kFetch) {
@@ -2116,7 +2136,7 @@ bz_integrate_kernel(const KParams P) {
                                 // the network proposes each lane's level; the warp takes the
                                 // finest one (dead lanes propose level 0)
                                 float f[kMlpIn];
-                                mlp_features(kfeat, gslot[DYA - 2], gslot[DYA - 1], S, -double(level), f);
+                                mlp_features(kfeat, slot[DYA - 2], slot[DYA - 1], S, -double(level), f);
                                 const float T = mlp_warp_infer(P.mlp, f, mlp_stage + wib * kMlpWarpStage);
                                 int want = dead ? 0 : (int)ceilf(T + __ldg(&P.mlp->level_margin));
                                 want = want < 0 ? 0 : (want > kLevelMax ? kLevelMax : want);
@@ -2124,9 +2144,39 @@ bz_integrate_kernel(const KParams P) {
                             }
                         }
                         int L = level, qpos = 0;
-                        const bool from_floor = level == 0;
                         bool fallback = false, coarse_end = false, refined = false;
-                        for (;;) {
+                        bool done = false;
+                        const bool from_floor = level == 0;
+                        if (from_floor) {
+                            // one step over the interval, stage values from the
+                            // record in shared memory: where nearly all intervals of
+                            // a floor workload begin and end (a copy of the attempt
+                            // without the level arithmetic, the coarsening test and
+                            // the table's address: honeycomb 1024 x 1024, mixed, 5.82
+                            // -> 5.30 ms for 256 intervals with the rest of the path)
+                            bool ok = true;
+                            double xn[3], e[3], k0[3];
+                            const TableEval<NF, R, table_values<M, R>()> tev{
+                                reinterpret_cast<const V *>(slot + DYA)};
+                            rkf78_attempt<M, NF, R>(ms, tev, t0, span, S, xn, e, k0);
+#pragma unroll
+                            for (int c = 0; c < 3; ++c)
+                                ok = ok && !(fabs(e[c]) > error_den<M, R>(P, S[c], k0[c], span));
+                            if (!dead) ++my_attempts;
+                            done = __all_sync(kFull, ok || dead);
+                            if (done) {
+                                if (!dead) {
+                                    S[0] = xn[0];
+                                    S[1] = xn[1];
+                                    S[2] = xn[2];
+                                }
+                            } else {
+                                if (!dead && !ok) ++my_rejects;
+                                refined = true;
+                                L = 1;
+                            }
+                        }
+                        while (!done) {
                             const double h = span * pow2_neg(L);
                             const double tq = t0 + qpos * h;
                             bool ok = true, small = true;

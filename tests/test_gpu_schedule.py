@@ -61,3 +61,18 @@ def test_schedules(engine, n_sub, tol):
     # tolerances a decision on a threshold may differ and then moves j by the tolerance
     assert rel_l2(j, jr) <= max(TOL, 0.01 * tol[1])
     assert abs(st.attempted_steps - st_o.attempted) <= 2e-3 * st_o.attempted
+
+
+@pytest.mark.parametrize("precision,n_meas", [(api.PREC_FP64, n) for n in (1, 7, 8, 9, 17, 64)] +
+                         [(api.PREC_MIXED, n) for n in (7, 8, 9, 17, 64)])
+@pytest.mark.parametrize("model", ["honeycomb", "dirac2d"])
+def test_dyadic_sample_blocks(engine, model, precision, n_meas):
+    """The dyadic steppers' blocks and records (rel_tol 1e-8; FP32 stages: 6e-8 of the
+    trajectories' size a step, so the mixed runs start at windows whose current has risen to
+    more than a millionth of it)."""
+    sys_, p, grid, _, jr, _ = _case(n_meas, 50, (1e-12, 1e-8), 9, 5, model=model)
+    j, _ = engine.current_density(sys_, p, grid,
+                                  api.solver(1e-12, 1e-8, precision=precision,
+                                             proposer=api.PROPOSER_LOCKSTEP))
+    bar = 1e-7 if precision == api.PREC_FP64 else 1e-5
+    assert np.all(np.isfinite(j)) and rel_l2(j, jr) <= bar
