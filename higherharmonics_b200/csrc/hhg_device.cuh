@@ -218,6 +218,7 @@ struct PulseDev {
     long long j_off;      // samples into j
     int n_meas;
     int items;            // work items of this pulse
+    int chunk_len;        // intervals per chunk (intervals in parallel)
     int kind;             // PulseKind
     int spline_n;         // SPLINE: samples (the coefficient array holds spline_n + 2)
     double gauss_c, gauss_2s2;         // GAUSS: centre and 2 sigma^2
@@ -257,7 +258,16 @@ struct KParams {
     double energy_cut;
     long long chan_stride;
     double *kout;
+    // intervals in parallel (chunk_propagator_kernel): the most chunks of any
+    // pulse, the propagators, and kChunkStat counters per pulse: the flag that
+    // discards its chunked run, its attempted and rejected steps.  only_discarded:
+    // the kernel integrates the pulses whose chunked run was discarded
+    double *prop;
+    int n_chunks;
+    unsigned long long *chunk_stat;
+    bool only_discarded;
 };
+constexpr int kChunkStat = 4;
 constexpr int kHistFields = 12;
 
 // ---------------------------------------------------------------------------
@@ -1294,10 +1304,10 @@ __device__ __forceinline__ void rkf78_attempt_unscaled(const ModelState<M, doubl
 // ---------------------------------------------------------------------------
 // One attempted Fehlberg 7(8) step (E. Fehlberg, NASA TR R-287, 1968):
 // 13 stages, the 8th-order solution propagated, error = b8 - b7 =
-// 41/840 (k12 + k13 - k1 - k11).  R is the stage precision; the state, the
-// solution increment and the error estimate are FP64.
+// 41/840 (k12 + k13 - k1 - k11), in FP64 for NV states of one k-point (one, or
+// the three basis vectors of a propagator).
 //
-// FP64: the kernel is bound by its FP64 instructions, so they are what this
+// The kernel is bound by its FP64 instructions, so they are what this
 // form saves.  The stages hold h k (the step size multiplies the model's
 // constants once), which makes every stage value one FMA chain from the
 // state, without a product by h and without joining partial sums, and makes
@@ -1307,8 +1317,70 @@ __device__ __forceinline__ void rkf78_attempt_unscaled(const ModelState<M, doubl
 // waits.  The error comes back as h (k12 + k13 - k1 - k11): the controller's
 // tolerances carry the factor 840/41.  Pi-flux 2D, 256 x 256, 8192 intervals:
 // 430 -> 366 FP64 instructions a step, 87.4 -> 76.6 ms.
-// Outputs: xn, e (scaled form: without 41/840) and k0 (scaled form: times h).
+// Outputs: xn, e (without 41/840) and k0 (times h).
 // ---------------------------------------------------------------------------
+template <int M, int NF, int NV, class Eval>
+__device__ __forceinline__ void rkf78_attempt_scaled(const ModelState<M, double> &ms, const Eval &ev,
+                                                     double t, double h, const double (&x)[NV][3],
+                                                     double (&xn)[NV][3], double (&e)[NV][3],
+                                                     double (&k0d)[NV][3]) {
+    using Node = typename ModelState<M, double>::Node;
+    double k[NV][13][3], f[NF];
+    const auto st = ms.step(h);
+    ev(0, t, f);
+    const Node n0 = ms.node(st, f);
+    Node n3 = n0, n10 = n0;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) ms.eval(st, n0, x[v], k[v][0]);
+#define HHG_STAGE(s, CHAIN)                                                         \
+    {                                                                               \
+        Node nd = s == 7 ? n3 : s == 11 ? n0 : n10;                                 \
+        if constexpr (s != 7 && s != 11 && s != 12) {                               \
+            ev(s, t + rk_c(s) * h, f);                                              \
+            nd = ms.node(st, f);                                                    \
+            if constexpr (s == 3) n3 = nd;                                          \
+            if constexpr (s == 10) n10 = nd;                                        \
+        }                                                                           \
+        _Pragma("unroll") for (int v = 0; v < NV; ++v) {                            \
+            double xt[3];                                                           \
+            _Pragma("unroll") for (int i = 0; i < 3; ++i) xt[i] = CHAIN;            \
+            ms.eval(st, nd, xt, k[v][s]);                                           \
+        }                                                                           \
+    }
+#define K(c, j, acc) fma(c, k[v][j][i], acc)
+    HHG_STAGE(1, K(2.0 / 27.0, 0, x[v][i]))
+    HHG_STAGE(2, K(1.0 / 12.0, 1, K(1.0 / 36.0, 0, x[v][i])))
+    HHG_STAGE(3, K(1.0 / 8.0, 2, K(1.0 / 24.0, 0, x[v][i])))
+    HHG_STAGE(4, K(25.0 / 16.0, 3, K(-25.0 / 16.0, 2, K(5.0 / 12.0, 0, x[v][i]))))
+    HHG_STAGE(5, K(1.0 / 5.0, 4, K(1.0 / 4.0, 3, K(1.0 / 20.0, 0, x[v][i]))))
+    HHG_STAGE(6, K(125.0 / 54.0, 5, K(-65.0 / 27.0, 4, K(125.0 / 108.0, 3, K(-25.0 / 108.0, 0, x[v][i])))))
+    HHG_STAGE(7, K(13.0 / 900.0, 6, K(-2.0 / 9.0, 5, K(61.0 / 225.0, 4, K(31.0 / 300.0, 0, x[v][i])))))
+    HHG_STAGE(8, K(3.0, 7, K(67.0 / 90.0, 6, K(-107.0 / 9.0, 5, K(704.0 / 45.0, 4,
+              K(-53.0 / 6.0, 3, K(2.0, 0, x[v][i])))))))
+    HHG_STAGE(9, K(-1.0 / 12.0, 8, K(17.0 / 6.0, 7, K(-19.0 / 60.0, 6, K(311.0 / 54.0, 5,
+              K(-976.0 / 135.0, 4, K(23.0 / 108.0, 3, K(-91.0 / 108.0, 0, x[v][i]))))))))
+    HHG_STAGE(10, K(18.0 / 41.0, 9, K(45.0 / 164.0, 8, K(45.0 / 82.0, 7, K(2133.0 / 4100.0, 6,
+               K(-301.0 / 82.0, 5, K(4496.0 / 1025.0, 4, K(-341.0 / 164.0, 3, K(2383.0 / 4100.0, 0, x[v][i])))))))))
+    HHG_STAGE(11, K(6.0 / 41.0, 9, K(3.0 / 41.0, 8, K(-3.0 / 41.0, 7, K(-3.0 / 205.0, 6,
+               K(-6.0 / 41.0, 5, K(3.0 / 205.0, 0, x[v][i])))))))
+    HHG_STAGE(12, K(1.0, 11, K(12.0 / 41.0, 9, K(33.0 / 164.0, 8, K(51.0 / 82.0, 7, K(2193.0 / 4100.0, 6,
+               K(-289.0 / 82.0, 5, K(4496.0 / 1025.0, 4, K(-341.0 / 164.0, 3, K(-1777.0 / 4100.0, 0, x[v][i]))))))))))
+#undef K
+#undef HHG_STAGE
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const double k1112 = k[v][11][i] + k[v][12][i];
+            xn[v][i] = x[v][i] + (34.0 / 105.0 * k[v][5][i] + 9.0 / 35.0 * (k[v][6][i] + k[v][7][i]) +
+                                  9.0 / 280.0 * (k[v][8][i] + k[v][9][i]) + 41.0 / 840.0 * k1112);
+            e[v][i] = k1112 - (k[v][0][i] + k[v][10][i]);
+            k0d[v][i] = k[v][0][i];
+        }
+}
+
+// One attempt in precision R of the stages; outputs xn, e and k0 (scaled
+// attempts: as above).
 template <int M, int NF, typename R, class Eval>
 __device__ __forceinline__ void rkf78_attempt(const ModelState<M, R> &ms, const Eval &ev,
                                               double t, double h, const double *x, double *xn,
@@ -1318,54 +1390,14 @@ __device__ __forceinline__ void rkf78_attempt(const ModelState<M, R> &ms, const 
     } else if constexpr (Traits<M>::kStart) {
         rkf78_attempt_unscaled<M, NF>(ms, ev, t, h, x, xn, e, k0d);
     } else {
-        using Node = typename ModelState<M, R>::Node;
-        double k[13][3], f[NF];
-        const auto st = ms.step(h);
-        ev(0, t, f);
-        const Node n0 = ms.node(st, f);
-        Node n3 = n0, n10 = n0;
-        ms.eval(st, n0, x, k[0]);
-#define HHG_STAGE(s, CHAIN)                                                         \
-    {                                                                               \
-        double xt[3];                                                               \
-        _Pragma("unroll") for (int i = 0; i < 3; ++i) xt[i] = CHAIN;                \
-        if constexpr (s == 7 || s == 11 || s == 12) {                               \
-            ms.eval(st, s == 7 ? n3 : s == 11 ? n0 : n10, xt, k[s]);                \
-        } else {                                                                    \
-            ev(s, t + rk_c(s) * h, f);                                              \
-            const Node nd = ms.node(st, f);                                      \
-            if constexpr (s == 3) n3 = nd;                                          \
-            if constexpr (s == 10) n10 = nd;                                        \
-            ms.eval(st, nd, xt, k[s]);                                              \
-        }                                                                           \
-    }
-#define K(c, j, acc) fma(c, k[j][i], acc)
-        HHG_STAGE(1, K(2.0 / 27.0, 0, x[i]))
-        HHG_STAGE(2, K(1.0 / 12.0, 1, K(1.0 / 36.0, 0, x[i])))
-        HHG_STAGE(3, K(1.0 / 8.0, 2, K(1.0 / 24.0, 0, x[i])))
-        HHG_STAGE(4, K(25.0 / 16.0, 3, K(-25.0 / 16.0, 2, K(5.0 / 12.0, 0, x[i]))))
-        HHG_STAGE(5, K(1.0 / 5.0, 4, K(1.0 / 4.0, 3, K(1.0 / 20.0, 0, x[i]))))
-        HHG_STAGE(6, K(125.0 / 54.0, 5, K(-65.0 / 27.0, 4, K(125.0 / 108.0, 3, K(-25.0 / 108.0, 0, x[i])))))
-        HHG_STAGE(7, K(13.0 / 900.0, 6, K(-2.0 / 9.0, 5, K(61.0 / 225.0, 4, K(31.0 / 300.0, 0, x[i])))))
-        HHG_STAGE(8, K(3.0, 7, K(67.0 / 90.0, 6, K(-107.0 / 9.0, 5, K(704.0 / 45.0, 4,
-                  K(-53.0 / 6.0, 3, K(2.0, 0, x[i])))))))
-        HHG_STAGE(9, K(-1.0 / 12.0, 8, K(17.0 / 6.0, 7, K(-19.0 / 60.0, 6, K(311.0 / 54.0, 5,
-                  K(-976.0 / 135.0, 4, K(23.0 / 108.0, 3, K(-91.0 / 108.0, 0, x[i]))))))))
-        HHG_STAGE(10, K(18.0 / 41.0, 9, K(45.0 / 164.0, 8, K(45.0 / 82.0, 7, K(2133.0 / 4100.0, 6,
-                   K(-301.0 / 82.0, 5, K(4496.0 / 1025.0, 4, K(-341.0 / 164.0, 3, K(2383.0 / 4100.0, 0, x[i])))))))))
-        HHG_STAGE(11, K(6.0 / 41.0, 9, K(3.0 / 41.0, 8, K(-3.0 / 41.0, 7, K(-3.0 / 205.0, 6,
-                   K(-6.0 / 41.0, 5, K(3.0 / 205.0, 0, x[i])))))))
-        HHG_STAGE(12, K(1.0, 11, K(12.0 / 41.0, 9, K(33.0 / 164.0, 8, K(51.0 / 82.0, 7, K(2193.0 / 4100.0, 6,
-                   K(-289.0 / 82.0, 5, K(4496.0 / 1025.0, 4, K(-341.0 / 164.0, 3, K(-1777.0 / 4100.0, 0, x[i]))))))))))
-#undef K
-#undef HHG_STAGE
+        const double x1[1][3] = {{x[0], x[1], x[2]}};
+        double xn1[1][3], e1[1][3], k1[1][3];
+        rkf78_attempt_scaled<M, NF, 1>(ms, ev, t, h, x1, xn1, e1, k1);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            const double k1112 = k[11][i] + k[12][i];
-            xn[i] = x[i] + (34.0 / 105.0 * k[5][i] + 9.0 / 35.0 * (k[6][i] + k[7][i]) +
-                            9.0 / 280.0 * (k[8][i] + k[9][i]) + 41.0 / 840.0 * k1112);
-            e[i] = k1112 - (k[0][i] + k[10][i]);
-            k0d[i] = k[0][i];
+            xn[i] = xn1[0][i];
+            e[i] = e1[0][i];
+            k0d[i] = k1[0][i];
         }
     }
 }
@@ -1416,9 +1448,7 @@ __device__ __forceinline__ void rotation_factors(double x, double &sa, double &c
 }
 
 // Rodrigues rotation S <- exp([w]_x) S.
-__device__ __forceinline__ void rotate(const double *w, double *S) {
-    double sa, ca;
-    rotation_factors(w[0] * w[0] + w[1] * w[1] + w[2] * w[2], sa, ca);
+__device__ __forceinline__ void rotate(const double *w, double sa, double ca, double *S) {
     const double wx0 = w[1] * S[2] - w[2] * S[1];
     const double wx1 = w[2] * S[0] - w[0] * S[2];
     const double wx2 = w[0] * S[1] - w[1] * S[0];
@@ -1428,6 +1458,11 @@ __device__ __forceinline__ void rotate(const double *w, double *S) {
     S[0] += sa * wx0 + ca * ww0;
     S[1] += sa * wx1 + ca * ww1;
     S[2] += sa * wx2 + ca * ww2;
+}
+__device__ __forceinline__ void rotate(const double *w, double *S) {
+    double sa, ca;
+    rotation_factors(w[0] * w[0] + w[1] * w[1] + w[2] * w[2], sa, ca);
+    rotate(w, sa, ca, S);
 }
 
 // The reference's Dirac-3D Magnus step (DiracSystem.cpp:190-210): with the
@@ -1748,10 +1783,10 @@ constexpr int kFreeWindow = 8;
 // butterfly per sample costs ten shuffles and five additions in a row (175
 // cycles).  A fixed order.  Rows are padded to 33 doubles (bank conflicts).
 constexpr int kRing = 8, kRingRow = 33;
-__device__ __forceinline__ void put_sample(int i, double c, int N, int sub, int lane, double *ring,
+__device__ __forceinline__ void put_sample(int i, double c, int last, int sub, int lane, double *ring,
                                            double *prow) {
     ring[(i & (kRing - 1)) * kRingRow + lane] = c;
-    if ((i & (kRing - 1)) != kRing - 1 && i != N) return;
+    if ((i & (kRing - 1)) != kRing - 1 && i != last) return;
     __syncwarp();
     const int s = lane & (kRing - 1), part = lane / kRing;
     const double *r = ring + s * kRingRow + part * (32 / 4);
@@ -1860,6 +1895,150 @@ __device__ void integrate_free(const KParams &P, const PulseDev &pd, const Model
     }
 }
 
+// ---------------------------------------------------------------------------
+// Intervals in parallel.  On a small grid a run is a serial chain of intervals
+// on a few warps while the chip idles (8 x 8 k-points: 2 warps, 4096 steps in
+// a row).  The equations are linear in S and, on the standard schedule, the
+// steps do not depend on it, so the run splits into chunks of intervals:
+//   1. every chunk's propagator, one warp per (tile, chunk): the three basis
+//      vectors through the chunk's standard steps (the right-hand side's
+//      momentum part is shared by the three);
+//   2. the run itself (bz_integrate_kernel, CHUNK), every chunk from the state
+//      that the propagators before it give, with the full controller.  It is
+//      the sequential run up to rounding as long as the standard schedule
+//      holds: each chunk's end state is compared with its propagator's
+//      (kChunkTol), and a difference, a failed trajectory or an error estimate
+//      beyond the schedule's bounds discards the pulse's chunked run;
+//   3. the sequential kernel, for the pulses whose chunked run was discarded.
+// About 3.5 times the arithmetic over n_chunks times the warps: 8 x 8 k-points
+// over 1024 intervals 2.2 -> 0.085 ms (sequential -> in parallel), 64 x 64 over
+// 4096 9.0 -> 5.4 ms, with Magnus-4 3.2 -> 0.33 ms.
+// ---------------------------------------------------------------------------
+constexpr double kChunkTol = 1e-12;
+__device__ __forceinline__ void discard_chunks(const KParams &P, int pulse) {
+    *(volatile unsigned long long *)(P.chunk_stat + kChunkStat * pulse) = 1ull;
+}
+// (one lane reads: the same answer for the warp)
+__device__ __forceinline__ bool chunk_discarded(const KParams &P, int pulse, int lane) {
+    unsigned off = 0;
+    if (lane == 0) off = *(volatile unsigned long long *)(P.chunk_stat + kChunkStat * pulse) != 0ull;
+    return __shfl_sync(kFull, off, 0) != 0;
+}
+__device__ __forceinline__ double *propagator(const KParams &P, long long item, int chunk, int lane) {
+    return P.prop + ((size_t)item * P.n_chunks + chunk) * (9 * 32) + lane;
+}
+// S <- P_chunk S; column v of the propagator is the image of basis vector v
+__device__ __forceinline__ void apply_propagator(const KParams &P, long long item, int chunk, int lane,
+                                                 double *S) {
+    const double *m = propagator(P, item, chunk, lane);
+    double o[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) o[i] = m[32 * i] * S[0] + m[32 * (3 + i)] * S[1] + m[32 * (6 + i)] * S[2];
+    S[0] = o[0];
+    S[1] = o[1];
+    S[2] = o[2];
+}
+
+template <int M, int D, int STEPPER>
+__global__ void __launch_bounds__(kBlockThreads, 4) chunk_propagator_kernel(const KParams P) {
+    constexpr int NF = Traits<M>::NF;
+    constexpr int SLOT = slot_doubles(NF, D);
+    constexpr int SCHED = slot_sched(NF, D);
+    constexpr int TAB = slot_table(NF, D);
+    constexpr int COPY = STEPPER == 1 ? slot_poly(NF) + 2 * NF : SLOT;
+    static_assert(STEPPER == 0 || STEPPER == 1, "RKF78 or Magnus-4");
+    __shared__ __align__(16) double stage[kWarpsPerBlock][2][COPY];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    // chunks 0 .. n_chunks - 2 of every item (the last one leads nowhere)
+    const long long id = blockIdx.x * (long long)kWarpsPerBlock + wib;
+    const long long item = id / (P.n_chunks - 1);
+    const int chunk = (int)(id % (P.n_chunks - 1));
+    if (item >= P.n_items) return;
+    const int tile = (int)(item % P.items_per_pulse);
+    const int p = (int)(item / P.items_per_pulse);
+    const PulseDev &pd = P.pulses[p];
+    const int i0 = chunk * pd.chunk_len, i1 = i0 + pd.chunk_len;
+    if (i1 > pd.n_meas) return;  // the pulse ends in this chunk
+    const double *coef = P.coef + pd.coef_off;
+    const int q = tile * 32 + lane;
+    const bool valid = q < P.n_k;
+    double row[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) row[c] = valid ? __ldg(P.ktab + (size_t)q * 8 + c) : 0.0;
+    if (!valid) row[2] = 1.0;
+    ModelState<M, double> ms;
+    ms.init(pd, row);
+    double x[3][3] = {{1.0, 0.0, 0.0}, {0.0, 1.0, 0.0}, {0.0, 0.0, 1.0}};
+    // any state of length 1 has an error below the norm over the three columns
+    const double tol = P.abs_tol + 2.0 * P.rel_tol;
+    auto fetch = [&](int i) {
+        const double *src = coef + (size_t)i * SLOT;
+        for (int c = lane; c < COPY / 2; c += 32) copy16_async(stage[wib][i & 1] + 2 * c, src + 2 * c);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(i0);
+    for (int i = i0; i < i1; ++i) {
+        const double *slot = stage[wib][i & 1];
+        __syncwarp();  // the other buffer has been read
+        if (i + 1 < i1) {
+            fetch(i + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncwarp();
+        const double t0 = slot[0], t1 = slot[1];
+        if constexpr (STEPPER == 1) {
+            const int ns = P.magnus_substeps;
+            const double hs = ns == 1 ? t1 - t0 : (t1 - t0) / ns;
+            double f[2 * NF];
+#pragma unroll
+            for (int n = 0; n < 2 * NF; ++n) f[n] = slot[slot_poly(NF) + n];
+            for (int s = 0;;) {
+                double w[3], sa, ca;
+                ms.omega(hs, f, f + NF, w);
+                rotation_factors(w[0] * w[0] + w[1] * w[1] + w[2] * w[2], sa, ca);
+#pragma unroll
+                for (int v = 0; v < 3; ++v) rotate(w, sa, ca, x[v]);
+                if (++s == ns) break;
+                load_even<2 * NF>(coef + (size_t)i * SLOT + slot_poly(NF) + s * (2 * NF), f);
+            }
+        } else {
+            const int n_std = (int)slot[SCHED];
+            bool off = true;  // until the last tabulated step reaches t1
+#pragma unroll 1
+            for (int wa = 0; wa < n_std; ++wa) {
+                const double ts = slot[SCHED + 2 + wa], h = slot[SCHED + 2 + kMaxStd + wa];
+                const TableEval<NF, double> ev{slot + TAB + wa * 13 * NF};
+                double xn[3][3], e[3][3], k0[3][3];
+                rkf78_attempt_scaled<M, NF, 3>(ms, ev, ts, h, x, xn, e, k0);
+                const bool last = !(t1 - (ts + h) > kDblEps);
+                const double bound = (last ? 1.0 : wa == n_std - 2 ? slot[SCHED + 1] : P.err_floor) * tol;
+                bool beyond = false;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    beyond = beyond || !(e[0][c] * e[0][c] + e[1][c] * e[1][c] + e[2][c] * e[2][c] <= bound * bound);
+#pragma unroll
+                    for (int v = 0; v < 3; ++v) x[v][c] = xn[v][c];
+                }
+                off = beyond || !last;
+                if (beyond) break;
+            }
+            const bool stop = __any_sync(kFull, valid && off);
+            if (stop && lane == 0) discard_chunks(P, p);
+            if (stop || ((i & 7) == 0 && chunk_discarded(P, p, lane))) {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                return;
+            }
+        }
+    }
+    double *m = propagator(P, item, chunk, lane);
+#pragma unroll
+    for (int v = 0; v < 3; ++v)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) m[32 * (3 * v + c)] = x[v][c];
+}
+
 constexpr int kLevelMax = 10;
 // 2^-L for 0 <= L <= 1022, exactly: the dyadic step span * 2^-L equals
 // ldexp(span, -L) without its range handling
@@ -1905,7 +2084,23 @@ __host__ __device__ constexpr int min_blocks(int model, bool fp64, int stepper) 
 //   integrand of DiracSystem::compute_current_density,
 //   DiracSystem.cpp:300-311; dead trajectories give 0 and are counted).
 // OUT 1-3 are built for the PiFlux models only, OUT 4 for the Dirac-3D ones.
-template <int M, int D, typename R, int STEPPER, int PROPOSER, int OUT = 0>
+// A warp's attempted and rejected steps into counters [1] and [2].
+__device__ __forceinline__ void add_steps(unsigned long long *counters, unsigned long long attempts,
+                                          unsigned long long rejects, int lane) {
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        attempts += __shfl_xor_sync(kFull, attempts, o);
+        rejects += __shfl_xor_sync(kFull, rejects, o);
+    }
+    if (lane == 0) {
+        atomicAdd(counters + 1, attempts);
+        atomicAdd(counters + 2, rejects);
+    }
+}
+
+// CHUNK: an item is one chunk of a tile's intervals, started from the state
+// that the propagators of the chunks before it give (chunk_propagator_kernel).
+template <int M, int D, typename R, int STEPPER, int PROPOSER, int OUT = 0, bool CHUNK = false>
 __global__ void __launch_bounds__(kBlockThreads, min_blocks(M, sizeof(R) == sizeof(double), STEPPER))
 bz_integrate_kernel(const KParams P) {
     constexpr int NF = Traits<M>::NF;
@@ -1950,16 +2145,34 @@ bz_integrate_kernel(const KParams P) {
     const int wib = threadIdx.x >> 5;
     double *slot = stage_raw[wib][0];
 
+    static_assert(!CHUNK || (!kNarrow && kFetch && PROPOSER == 0 && OUT != 1), "chunked variants");
+    __shared__ double chunk_s0[kWarpsPerBlock][CHUNK ? 96 : 1];  // the chunk's start state
+
     unsigned long long my_attempts = 0, my_rejects = 0;
     for (;;) {
         long long item = 0;
         if (lane == 0) item = (long long)atomicAdd(P.counters, 1ull);
         item = __shfl_sync(kFull, item, 0);
         if (item >= P.n_items) break;
+        int chunk = 0;
+        if constexpr (CHUNK) {
+            chunk = (int)(item % P.n_chunks);
+            item /= P.n_chunks;
+        }
         const int p = (int)(item / P.items_per_pulse);
+        if (CHUNK || P.only_discarded) {
+            const bool off = chunk_discarded(P, p, lane);
+            if (CHUNK ? off : !off) continue;
+        }
         const int tile = (int)(item % P.items_per_pulse);
         const PulseDev &pd = P.pulses[p];
         const int N = pd.n_meas;
+        // this item's first sample, its last interval's end and its last sample
+        const int i0 = CHUNK ? chunk * pd.chunk_len : 0;
+        if (CHUNK && chunk > 0 && i0 >= N) continue;
+        const bool to_end = !CHUNK || N - i0 <= pd.chunk_len;
+        const int i_end = to_end ? N : i0 + pd.chunk_len;
+        const int i_last = to_end ? N : i_end - 1;
         const double dt0 = pd.dt0;
         const double tb = pd.t_begin, te = pd.t_end;
         double *prow = P.part + pd.part_off + (long long)tile * (N + 1);
@@ -1996,9 +2209,15 @@ bz_integrate_kernel(const KParams P) {
                 for (int c = 0; c < 4; ++c) mom_next[c] = __ldg(coef + TAB + c);
             }
 
+            if constexpr (CHUNK) {
+                for (int c = 0; c < chunk; ++c) apply_propagator(P, item, c, lane, S);
+#pragma unroll
+                for (int e = 0; e < 3; ++e) chunk_s0[wib][32 * e + lane] = S[e];
+            }
+
             // (one running pointer per 32 pieces of 16 bytes)
             constexpr int kPieces = (COPY / 2 + 31) / 32;
-            const double *fsrc = coef + 2 * lane;
+            const double *fsrc = coef + 2 * lane + (CHUNK ? (size_t)i0 * SLOT : 0);
             auto fetch = [&](int interval) {
                 double *dst = stage_raw[wib][interval & (kFetch ? 1 : 0)] + 2 * lane;
 #pragma unroll
@@ -2010,7 +2229,7 @@ bz_integrate_kernel(const KParams P) {
             };
             if constexpr (kFetch) {
                 __syncwarp();  // the previous tile's last record has been read
-                fetch(0);
+                fetch(i0);
             }
 
             if constexpr (kFree) {
@@ -2020,9 +2239,9 @@ bz_integrate_kernel(const KParams P) {
                 integrate_free<M, D>(P, pd, ms, coef, dt0, tb, te, N, w, dead, S, held, prow, sub, lane,
                                      free_ring[wib], my_attempts, my_rejects);
             } else {
-            for (int i = 0; i <= N; ++i) {
-                const double *rec = pd.s0rec;
-                if (i > 0) {
+            for (int i = i0; i <= i_end; ++i) {
+                const double *rec = CHUNK && i0 > 0 ? coef + (size_t)(i0 - 1) * SLOT + 4 : pd.s0rec;
+                if (i > i0) {
                     // interval i-1 in this warp's shared slot (the closed-form
                     // Magnus step reads its moments and the record straight from
                     // the staging table: warp broadcasts of a few values)
@@ -2030,7 +2249,7 @@ bz_integrate_kernel(const KParams P) {
                     if constexpr (kFetch) {
                         slot = stage_raw[wib][(i - 1) & 1];
                         __syncwarp();  // the other buffer has been read
-                        if (i < N) {
+                        if (i < i_end) {
                             fetch(i);
                             asm volatile("cp.async.wait_group 1;" ::: "memory");
                         } else {
@@ -2241,10 +2460,11 @@ bz_integrate_kernel(const KParams P) {
                         atomicMax(P.status, 3);
                     }
                 }
+                if (CHUNK && i > i_last) break;  // the next chunk's first sample
                 // sample i at t_i = i * measure_every + t_begin (PiFlux.cpp:834-836)
                 if constexpr (OUT == 0) {
                     const double c = dead ? 0.0 : w * ms.vertex(rec, S);
-                    if constexpr (kRingSum) put_sample(i, c, N, sub, lane, ring[wib], prow);
+                    if constexpr (kRingSum) put_sample(i, c, i_last, sub, lane, ring[wib], prow);
                     else keep_sample(i, warp_sum(c), N, sub, lane, held, prow);
                 } else if constexpr (OUT == 1) {
                     double c_lo = 0.0, c_hi = 0.0;
@@ -2287,18 +2507,28 @@ bz_integrate_kernel(const KParams P) {
                     }
                 }
             }
+            if constexpr (CHUNK) {
+                if (!to_end) {
+                    // the next chunk started from this chunk's propagator
+                    double v[3];
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) v[e] = chunk_s0[wib][32 * e + lane];
+                    apply_propagator(P, item, chunk, lane, v);
+                    const double tol = kChunkTol * (fabs(S[0]) + fabs(S[1]) + fabs(S[2]));
+                    const bool same = fabs(S[0] - v[0]) <= tol && fabs(S[1] - v[1]) <= tol &&
+                                      fabs(S[2] - v[2]) <= tol;
+                    if (valid && !same) discard_chunks(P, p);
+                }
+                if (valid && dead) discard_chunks(P, p);
+            }
             }  // interval-synchronous loop
         }
+        if constexpr (CHUNK) {
+            add_steps(P.chunk_stat + kChunkStat * p, my_attempts, my_rejects, lane);
+            my_attempts = my_rejects = 0;
+        }
     }
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-        my_attempts += __shfl_xor_sync(kFull, my_attempts, o);
-        my_rejects += __shfl_xor_sync(kFull, my_rejects, o);
-    }
-    if (lane == 0) {
-        atomicAdd(P.counters + 1, my_attempts);
-        atomicAdd(P.counters + 2, my_rejects);
-    }
+    add_steps(P.counters, my_attempts, my_rejects, lane);
 }
 
 // ---------------------------------------------------------------------------

@@ -62,6 +62,11 @@ struct hhg_plan {
     int n_pulses = 0;
     int64_t n_k = 0;
     int tiles_per_item = 1, items_per_pulse = 0;
+    // intervals in parallel (n_chunks > 1: the most of any pulse) and the
+    // chunks' propagators
+    int n_chunks = 1;
+    double *d_prop = nullptr;
+    unsigned long long *d_chunk_stat = nullptr;  // hhg::kChunkStat per pulse
     long long n_items = 0;
     long long j_len = 0, part_len = 0, coef_len = 0, n_intervals = 0;
     std::vector<PulseDev> pulses;
@@ -936,6 +941,46 @@ hhg_status check_relax(hhg_ctx *ctx, const hhg_system_desc &s, const hhg_pulse_d
     return HHG_OK;
 }
 
+// Intervals in parallel for plans of at most one 32-row tile per SM.  The
+// chunked run does about 3.5 times the arithmetic of the sequential one (the
+// three basis vectors, then the run); one warp alone keeps its scheduler's
+// FP64 pipe 40-80 % busy, so T tiles break even near T = 256 of the 592
+// schedulers (gapped Dirac, 4096 intervals: T = 32 9.0 -> 1.3 ms, T = 145 9.0
+// -> 5.9 ms).  A pulse's chunks, for about 12 warps per SM (4 lose 10-25 %) and
+// a multiple of the sample block, follow from its own tiles and intervals
+// alone, so pulses agree bit for bit with their single runs in every plan that
+// runs in chunks.
+constexpr int kChunkWarpsPerSm = 12, kMaxChunks = 128, kMinChunks = 4;
+void setup_chunks(hhg_plan *pl) {
+    pl->n_chunks = 1;
+    cudaFree(pl->d_prop);
+    cudaFree(pl->d_chunk_stat);
+    pl->d_prop = nullptr;
+    pl->d_chunk_stat = nullptr;
+    const hhg_ctx *ctx = pl->ctx;
+    int most = 1;
+    for (PulseDev &d : pl->pulses) {
+        const int want = (int)std::min<long long>((long long)kChunkWarpsPerSm * ctx->sm_count / std::max(pl->items_per_pulse, 1),
+                                                  std::min(d.n_meas / hhg::kRing, kMaxChunks));
+        d.chunk_len = want < kMinChunks ? d.n_meas
+                                        : ((d.n_meas + want - 1) / want + hhg::kRing - 1) / hhg::kRing * hhg::kRing;
+        most = std::max(most, (d.n_meas + d.chunk_len - 1) / d.chunk_len);
+    }
+    if (pl->tiles_per_item != 1 || pl->n_items > ctx->sm_count || most < kMinChunks ||
+        !hhg::chunk_variant(pl->model, pl->degree, pl->opts.precision, pl->opts.stepper,
+                            kernel_proposer(pl->opts.proposer), pl->opts.magnus_substeps, pl->out_mode))
+        return;
+    if (cudaMalloc(&pl->d_chunk_stat, sizeof(unsigned long long) * hhg::kChunkStat * pl->n_pulses) != cudaSuccess ||
+        cudaMalloc(&pl->d_prop, sizeof(double) * 9 * 32 * (size_t)pl->n_items * most) != cudaSuccess) {
+        cudaGetLastError();  // no room: the sequential run needs none
+        cudaFree(pl->d_chunk_stat);
+        pl->d_chunk_stat = nullptr;
+        pl->d_prop = nullptr;
+        return;
+    }
+    pl->n_chunks = most;
+}
+
 hhg_status launch_variant(const hhg_plan *pl, hhg::LaunchReq &r) {
     cudaError_t e = cudaErrorInvalidValue;
     switch (pl->model) {
@@ -1354,6 +1399,8 @@ static hhg_status plan_create_impl(hhg_ctx *ctx, const hhg_system_desc *sys,
         }
     }
 
+    setup_chunks(pl);
+
     auto fail = [&](const char *what, cudaError_t e) {
         hhg_plan_destroy(pl);
         return set_err(ctx, HHG_CUDA_ERROR, std::string(what) + ": " + cudaGetErrorString(e));
@@ -1464,6 +1511,8 @@ void hhg_plan_destroy(hhg_plan *pl) {
     cudaFree(pl->d_hist);
     cudaFree(pl->d_hist_count);
     cudaFree(pl->d_kout);
+    cudaFree(pl->d_prop);
+    cudaFree(pl->d_chunk_stat);
     if (pl->gexec) cudaGraphExecDestroy(pl->gexec);
     delete pl;
 }
@@ -1522,7 +1571,33 @@ hhg_status enqueue_integration(hhg_plan *pl, cudaStream_t s, bool events) {
     lr.stream = s;
     lr.occupancy_out = nullptr;
     if (events) HHG_CUDA(ctx, cudaEventRecord(ctx->ev[0], s));
-    hhg_status st = launch_variant(pl, lr);
+    hhg_status st = HHG_OK;
+    if (pl->n_chunks > 1) {
+        // the chunks' propagators, the chunked run, and the sequential run of the
+        // pulses whose chunked one was discarded
+        HHG_CUDA(ctx, cudaMemsetAsync(pl->d_chunk_stat, 0,
+                                      sizeof(unsigned long long) * hhg::kChunkStat * pl->n_pulses, s));
+        hhg::LaunchReq cr = lr;
+        cr.kp.prop = pl->d_prop;
+        cr.kp.n_chunks = pl->n_chunks;
+        cr.kp.chunk_stat = pl->d_chunk_stat;
+        auto ctas = [](long long warps) {
+            return (int)((warps + hhg::kWarpsPerBlock - 1) / hhg::kWarpsPerBlock);
+        };
+        cr.phase = 1;
+        cr.grid = ctas(pl->n_items * (pl->n_chunks - 1));
+        if ((st = launch_variant(pl, cr)) != HHG_OK) return st;
+        cr.phase = 2;
+        cr.kp.n_items = pl->n_items * pl->n_chunks;
+        cr.grid = ctas(cr.kp.n_items);
+        if ((st = launch_variant(pl, cr)) != HHG_OK) return st;
+        // the chunked run's failures are void: a failed trajectory discards it
+        HHG_CUDA(ctx, cudaMemsetAsync(pl->d_counters, 0, 8 * sizeof(unsigned long long), s));
+        HHG_CUDA(ctx, cudaMemsetAsync(pl->d_status, 0, sizeof(int), s));
+        lr.kp.chunk_stat = pl->d_chunk_stat;
+        lr.kp.only_discarded = true;
+    }
+    st = launch_variant(pl, lr);
     if (st != HHG_OK) return st;
     if (events) HHG_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
     // one reduction per output channel; k-resolved samples need none
@@ -1560,6 +1635,17 @@ hhg_status hhg_plan_fetch(hhg_plan *pl, double *j_out, hhg_stats *stats) {
     int status = 0;
     HHG_CUDA(ctx, cudaMemcpy(cnt, pl->d_counters, sizeof cnt, cudaMemcpyDeviceToHost));
     HHG_CUDA(ctx, cudaMemcpy(&status, pl->d_status, sizeof status, cudaMemcpyDeviceToHost));
+    if (pl->n_chunks > 1) {
+        // the steps of the pulses whose chunked run stands
+        std::vector<unsigned long long> cs((size_t)hhg::kChunkStat * pl->n_pulses);
+        HHG_CUDA(ctx, cudaMemcpy(cs.data(), pl->d_chunk_stat, cs.size() * sizeof cs[0], cudaMemcpyDeviceToHost));
+        for (int p = 0; p < pl->n_pulses; ++p) {
+            const unsigned long long *c = cs.data() + (size_t)hhg::kChunkStat * p;
+            if (c[0]) continue;
+            cnt[1] += c[1];
+            cnt[2] += c[2];
+        }
+    }
     if (j_out) HHG_CUDA(ctx, cudaMemcpy(j_out, pl->d_j, pl->j_len * sizeof(double), cudaMemcpyDeviceToHost));
     if (stats) {
         std::memset(stats, 0, sizeof *stats);
@@ -1934,7 +2020,7 @@ hhg_status hhg_learned_collect(hhg_ctx *ctx, const hhg_system_desc *sys,
                        "spline pulse too steep for the staged interpolants: its exact evaluation "
                        "runs the Brillouin-zone current only, without history recording");
     }
-    pl->record = true;
+    pl->record = true;  // (the carried step: no intervals in parallel)
     pl->hist_every = hist_every;
     pl->hist_cap = cap;
     cudaError_t e;
@@ -2035,6 +2121,7 @@ hhg_status retile(hhg_plan *pl, int tpi, long long ctas) {
     pl->tiles_per_item = tpi;
     pl->items_per_pulse = ipp;
     pl->n_items = (long long)ipp * pl->n_pulses;
+    setup_chunks(pl);
     HHG_CUDA(ctx, cudaMemcpy(pl->d_pulses, pl->pulses.data(), sizeof(PulseDev) * pl->n_pulses,
                              cudaMemcpyHostToDevice));
     const long long max_ctas = (long long)pl->occupancy * ctx->sm_count;
@@ -2191,6 +2278,7 @@ hhg_status output_plan(hhg_ctx *ctx, const hhg_system_desc *sys, const hhg_pulse
     };
     cudaError_t e;
     pl->out_mode = mode;
+    setup_chunks(pl);
     if (mode == 1) {  // a second channel of partial rows and of j
         cudaFree(pl->d_part);
         cudaFree(pl->d_j);
@@ -2385,6 +2473,7 @@ hhg_status dirac_quadrature(hhg_ctx *ctx, const hhg_system_desc *sys, const hhg_
                            "evaluation runs the Brillouin-zone current only");
         }
         np->out_mode = 4;
+        setup_chunks(np);  // none: the launches vary in size
         int occ = 0;
         hhg::LaunchReq lr{};
         lr.degree = np->degree;

@@ -19,6 +19,7 @@ struct LaunchReq {
     int *occupancy_out;  // blocks per SM for the selected variant (if non-null)
     int out_mode = 0;    // bz_integrate_kernel's OUT (1-3: PiFlux models, FP64, proposer 0/1;
                          // 4: Dirac-3D models, FP64, proposer 0)
+    int phase = 0;       // intervals in parallel: 1 the chunks' propagators, 2 the chunked run
 };
 
 struct StageReq {
@@ -37,9 +38,20 @@ struct StageReq {
     const double *gl30 = nullptr;  // layout 3: 30 nodes on [0, 1], then 30 weights (device)
 };
 
-template <int M, int D, typename R, int ST, int PR, int OUT = 0>
+// Variants with intervals in parallel: FP64, RKF78 on the reference schedule or
+// Magnus-4 from the staged sums, coherent models; the Brillouin-zone sum, and
+// the k-resolved outputs of PiFlux-3D.
+inline bool chunk_variant(int model, int degree, int precision, int stepper, int proposer, int substeps,
+                          int out_mode) {
+    const bool relax = model == PIFLUX3D_RELAX || model == HONEYCOMB_RELAX || model == DIRAC3D_RELAX;
+    return !relax && degree != 0 && precision == 0 &&
+           ((stepper == 0 && proposer == 0) || (stepper == 1 && substeps <= kMagnusTab)) &&
+           (out_mode == 0 || ((out_mode == 2 || out_mode == 3) && model == PIFLUX3D && stepper == 0));
+}
+
+template <int M, int D, typename R, int ST, int PR, int OUT = 0, bool CHUNK = false>
 cudaError_t launch_one(const LaunchReq &r) {
-    auto kern = bz_integrate_kernel<M, D, R, ST, PR, OUT>;
+    auto kern = bz_integrate_kernel<M, D, R, ST, PR, OUT, CHUNK>;
     const int dyn = PR == 3 ? mlp_smem_bytes() : 0;
     if (r.occupancy_out) {
         cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(r.occupancy_out, kern, kBlockThreads, dyn);
@@ -79,7 +91,29 @@ cudaError_t launch_out(const LaunchReq &r) {
 }
 
 template <int M, int D>
+cudaError_t launch_chunk(const LaunchReq &r) {
+    if constexpr (!Traits<M>::kRelax && D != 0) {
+        if (!chunk_variant(M, D, r.precision, r.stepper, r.proposer, r.kp.magnus_substeps, r.out_mode))
+            return cudaErrorNotSupported;
+        if (r.phase == 1) {
+            if (r.stepper == 1) chunk_propagator_kernel<M, D, 1><<<r.grid, kBlockThreads, 0, r.stream>>>(r.kp);
+            else chunk_propagator_kernel<M, D, 0><<<r.grid, kBlockThreads, 0, r.stream>>>(r.kp);
+            return cudaGetLastError();
+        }
+        if constexpr (M == PIFLUX3D) {
+            if (r.out_mode == 2) return launch_one<M, D, double, 0, 0, 2, true>(r);
+            if (r.out_mode == 3) return launch_one<M, D, double, 0, 0, 3, true>(r);
+        }
+        return r.stepper == 1 ? launch_one<M, D, double, 1, 0, 0, true>(r)
+                              : launch_one<M, D, double, 0, 0, 0, true>(r);
+    } else {
+        return cudaErrorNotSupported;
+    }
+}
+
+template <int M, int D>
 cudaError_t launch_deg(const LaunchReq &r) {
+    if (r.phase != 0) return launch_chunk<M, D>(r);
     if (r.out_mode != 0) return launch_out<M, D>(r);
     if constexpr (Traits<M>::kRelax) {
         // relaxation right-hand sides: FP64 controlled RKF78 only
@@ -134,7 +168,7 @@ cudaError_t launch_exact(const LaunchReq &r) {
 
 template <int M>
 cudaError_t launch_model(const LaunchReq &r) {
-    if (r.degree == 0) return launch_exact<M>(r);
+    if (r.degree == 0) return r.phase == 0 ? launch_exact<M>(r) : cudaErrorNotSupported;
     if (r.degree == 5) return launch_deg<M, 5>(r);
     if (r.degree == 7) return launch_deg<M, 7>(r);
     if (r.degree == 11) return launch_deg<M, 11>(r);
