@@ -155,8 +155,12 @@ __device__ __forceinline__ uint32_t kmaj_off(int row, int k, int rows) {
     return (uint32_t)((((k >> 3) * (rows >> 3) + (row >> 3)) << 7) + ((row & 7) << 4) + ((k & 7) << 1));
 }
 
-// SiLU(z) = z s and SiLU'(z) = s (1 + z (1 - s)) from one sigmoid s(z)
-__device__ __forceinline__ float sigmoid_f(float z) { return __frcp_rn(1.0f + __expf(-z)); }
+// SiLU(z) = z / (1 + e^-z) and SiLU'(z) = s (1 + z (1 - s)), s = 1 / (1 + e^-z)
+__device__ __forceinline__ float silu_f(float z, float &ds) {
+    const float d = 1.0f + __expf(-z), s = __frcp_rn(d);
+    ds = s * (1.0f + z * (1.0f - s));
+    return z / d;
+}
 
 // ---------------------------------------------------------------------------
 // Kernels
@@ -245,7 +249,7 @@ struct StepSmem {
     alignas(128) unsigned char w1[kH * kInPad * 2], w2[kH * kH * 2], w3[kH * kH * 2];
     alignas(128) unsigned char w2t[kH * kH * 2], w3t[kH * kH * 2];
     float b[3][kH], w4[kH];
-    float y[kColParts][kRows], gy[kRows], t[kRows];
+    float y[kRows], gy[kRows], t[kRows];
     float dw4[kH], db[3][kH], red[2][kStepThreads / 32];
     uint64_t mbar;
     uint32_t taddr;
@@ -396,7 +400,6 @@ __global__ void __launch_bounds__(kStepThreads) mlp_step_kernel(const bf16 *X, c
             }
         }
         // the hidden layers: Z_l stays in tensor memory, H_l goes to shared memory
-        float ys = quarter == 0 ? b4 : 0.0f;
 #pragma unroll 1
         for (int l = 0; l < 3; ++l) {
             before_products();
@@ -415,20 +418,29 @@ __global__ void __launch_bounds__(kStepThreads) mlp_step_kernel(const bf16 *X, c
                 tmem_ld8(trow + kColZ1 + kH * l + 8 * q, v);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
-                    const float z = v[c] + S.b[l][col + c], sg = sigmoid_f(z);
-                    v[c] = z * sg;
-                    ds[c] = sg * (1.0f + z * (1.0f - sg));
-                    // the output layer: each thread its columns of the row's dot product
-                    if (l == 2) ys += __bfloat162float(__float2bfloat16_rn(v[c])) * S.w4[col + c];
+                    v[c] = silu_f(v[c] + S.b[l][col + c], ds[c]);
                 }
                 if (GRAD) tmem_st8(trow + kColZ1 + kH * l + 8 * q, ds);
                 put8(h, ht, kH, row, col, v);
             }
         }
         if (!ok) break;
-        S.y[quarter][row] = ys;
-        __syncthreads();
-        const float y = (S.y[0][row] + S.y[1][row]) + (S.y[2][row] + S.y[3][row]);
+        // the output layer: the row's dot product in the order of the columns,
+        // handed on from quarter to quarter
+#pragma unroll 1
+        for (int qd = 0; qd < kColParts; ++qd) {
+            if (quarter == qd) {
+                float ys = qd == 0 ? b4 : S.y[row];
+#pragma unroll
+                for (int c = 0; c < kH / kColParts; ++c) {
+                    const int col = (kH / kColParts) * qd + c;
+                    ys += __bfloat162float(*reinterpret_cast<const bf16 *>(S.h3t + kmaj_off(col, row, kH))) * S.w4[col];
+                }
+                S.y[row] = ys;
+            }
+            __syncthreads();
+        }
+        const float y = S.y[row];
         if constexpr (!GRAD) {
             if (quarter == 0 && g < n) y_out[g] = y * out_sigma + out_mu;
         } else {
