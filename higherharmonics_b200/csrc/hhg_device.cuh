@@ -1421,25 +1421,28 @@ static __device__ __noinline__ double2 rotation_factors_large(double x) {
     sincos(th, &sn, &cs);
     return make_double2(sn / th, (1.0 - cs) / x);
 }
+__device__ __forceinline__ void rotation_series(double x, double &sa, double &ca) {
+    double s = 1.0 / 355687428096000.0, c = 1.0 / 6402373705728000.0;  // 1/17!, 1/18!
+    s = fma(s, x, -1.0 / 1307674368000.0);
+    c = fma(c, x, -1.0 / 20922789888000.0);
+    s = fma(s, x, 1.0 / 6227020800.0);
+    c = fma(c, x, 1.0 / 87178291200.0);
+    s = fma(s, x, -1.0 / 39916800.0);
+    c = fma(c, x, -1.0 / 479001600.0);
+    s = fma(s, x, 1.0 / 362880.0);
+    c = fma(c, x, 1.0 / 3628800.0);
+    s = fma(s, x, -1.0 / 5040.0);
+    c = fma(c, x, -1.0 / 40320.0);
+    s = fma(s, x, 1.0 / 120.0);
+    c = fma(c, x, 1.0 / 720.0);
+    s = fma(s, x, -1.0 / 6.0);
+    c = fma(c, x, -1.0 / 24.0);
+    sa = fma(s, x, 1.0);
+    ca = fma(c, x, 0.5);
+}
 __device__ __forceinline__ void rotation_factors(double x, double &sa, double &ca) {
     if (x <= 1.0) {
-        double s = 1.0 / 355687428096000.0, c = 1.0 / 6402373705728000.0;  // 1/17!, 1/18!
-        s = fma(s, x, -1.0 / 1307674368000.0);
-        c = fma(c, x, -1.0 / 20922789888000.0);
-        s = fma(s, x, 1.0 / 6227020800.0);
-        c = fma(c, x, 1.0 / 87178291200.0);
-        s = fma(s, x, -1.0 / 39916800.0);
-        c = fma(c, x, -1.0 / 479001600.0);
-        s = fma(s, x, 1.0 / 362880.0);
-        c = fma(c, x, 1.0 / 3628800.0);
-        s = fma(s, x, -1.0 / 5040.0);
-        c = fma(c, x, -1.0 / 40320.0);
-        s = fma(s, x, 1.0 / 120.0);
-        c = fma(c, x, 1.0 / 720.0);
-        s = fma(s, x, -1.0 / 6.0);
-        c = fma(c, x, -1.0 / 24.0);
-        sa = fma(s, x, 1.0);
-        ca = fma(c, x, 0.5);
+        rotation_series(x, sa, ca);
     } else {
         const double2 f = rotation_factors_large(x);
         sa = f.x;
@@ -1466,72 +1469,71 @@ __device__ __forceinline__ void rotate(const double *w, double *S) {
 }
 
 // The reference's Dirac-3D Magnus step (DiracSystem.cpp:190-210): with the
-// interval's Legendre moments m_q of A (Laser.cpp:40-55, staged per interval)
-// divided by |k|, Omega is the fourth-order Magnus series of
+// interval's Legendre moments of A (Laser.cpp:40-55, staged per interval)
+// divided by |k|, cf_q, Omega is the fourth-order Magnus series of
 // MagnusMatrix.cpp:25-57 for M(t) = H + A(t) A_k with H <-> h = (0, 0, 2|k| dt)
-// and A_k <-> (2 kappa dt, 0, -2 k_z dt).  For 3x3 skew matrices the
-// commutator is the cross product of the axial vectors, so each nested
-// commutator is a nested cross product; (a, b, c) of the reference's Omega
-// are (-w_2, w_1, -w_0), and U = exp(Omega) in the reference's closed form
-// (MagnusMatrix.cpp:59-75).
+// and A_k <-> v = (2 kappa dt, 0, -2 k_z dt).  For 3x3 skew matrices the
+// commutator is the cross product of the axial vectors; (a, b, c) of the
+// reference's Omega are (-w_2, w_1, -w_0), and U = exp(Omega).
 //
-// Every m_q of the series lies in the x-z plane (A_k has no y component and
-// h is along z), the cross product of two plane vectors lies along y, and
-// the cross product of a plane vector with a y vector lies in the plane
-// again; the nested cross products below are therefore evaluated on (x, z)
-// pairs and y scalars, forming none of the products with structural zeros
-// (which IEEE arithmetic would otherwise have to compute).
-struct XZ {
-    double x, z;
+// The series' vectors are m_1 = h + cf_0 v and m_q = cf_(q-1) v, so every
+// nested cross product reduces to few numbers: m_1 x m_q = cf_(q-1) K y with
+// K = (h x v)_y a constant of the trajectory, v x v = 0, and crossing a plane
+// vector m with y and back gives -|m|^2 y or the quarter turn m' = (-m_z,
+// m_x).  Collected (q = |m_1|^2, r = v . m_1, V = |v|^2, c = cf_1 K):
+//   plane part  (1 - c^2/7560) m_1 + (q cf_2 K / 2520) m_1'
+//               + K (-cf_1^2/60 - cf_2^2/420 + cf_1 cf_3/420 - q cf_1^2/2520) v'
+//   y part      K (-cf_1/6 - q cf_1/360 + q cf_3/840 - cf_1 cf_2 r/420
+//               + cf_1^3 V/840 - q^2 cf_1/15120)
+// -- the same series as the cross products one by one, in half the FP64
+// instructions.  U S is the rotation by w, its factors by their series at a
+// half or a quarter of the angle.
+struct DiracMagnus {
+    double inv, ks, kap, nkzs, K, V;
+    __device__ __forceinline__ DiracMagnus(double k_z, double kappa, double mk, double dt)
+        : inv(1.0 / mk), ks(2.0 * mk * dt), kap(2.0 * kappa * dt), nkzs(-(2.0 * k_z * dt)) {
+        K = ks * kap;
+        V = kap * kap + nkzs * nkzs;
+    }
+    __device__ __forceinline__ void omega(const double *mom, double *w) const {
+        const double c0 = mom[0] * inv, c1 = mom[1] * inv, c2 = mom[2] * inv, c3 = mom[3] * inv;
+        const double mx = c0 * kap, mz = fma(c0, nkzs, ks);
+        const double q = fma(mx, mx, mz * mz), r = fma(kap, mx, nkzs * mz);
+        const double c = c1 * K, c11 = c1 * c1;
+        const double em = fma(-c * c, 1.0 / 7560.0, 1.0);
+        const double ep = (q * c2) * (K * (1.0 / 2520.0));
+        const double ev = K * (fma(-1.0 / 60.0, c11, (1.0 / 420.0) * fma(c1, c3, -c2 * c2)) -
+                               (1.0 / 2520.0) * (q * c11));
+        w[0] = fma(em, mx, -fma(ep, mz, ev * nkzs));
+        w[2] = fma(em, mz, fma(ep, mx, ev * kap));
+        const double g = fma(q, fma(q, -1.0 / 15120.0, -1.0 / 360.0), -1.0 / 6.0);
+        w[1] = K * fma(c1, fma(c11, V * (1.0 / 840.0), fma(-1.0 / 420.0, c2 * r, g)), (1.0 / 840.0) * (q * c3));
+    }
 };
-// (u x v)_y of two plane vectors
-__device__ __forceinline__ double xz_cross(XZ u, XZ v) { return u.z * v.x - u.x * v.z; }
-// u x (0, y, 0)
-__device__ __forceinline__ XZ xz_cross_y(XZ u, double y) { return {-u.z * y, u.x * y}; }
-// (0, y, 0) x u
-__device__ __forceinline__ XZ y_cross_xz(double y, XZ u) { return {y * u.z, -y * u.x}; }
 
-__device__ __forceinline__ void dirac_magnus_step(double k_z, double kappa, double mk, double dt,
-                                                  const double *mom, double *S) {
-    const double inv = 1.0 / mk;
-    const double cf0 = mom[0] * inv, cf1 = mom[1] * inv, cf2 = mom[2] * inv, cf3 = mom[3] * inv;
-    const double ks = 2.0 * mk * dt, kap = 2.0 * kappa * dt, nkzs = -(2.0 * k_z * dt);
-    const XZ m1{cf0 * kap, ks + cf0 * nkzs};
-    const XZ m2{cf1 * kap, cf1 * nkzs}, m3{cf2 * kap, cf2 * nkzs}, m4{cf3 * kap, cf3 * nkzs};
-    const double c12 = xz_cross(m1, m2), c13 = xz_cross(m1, m3), c14 = xz_cross(m1, m4);
-    const XZ c112 = xz_cross_y(m1, c12), c113 = xz_cross_y(m1, c13);
-    double wx = m1.x, wy = -(c12 / 6.0), wz = m1.z;
-    auto plane = [&](double coef, XZ t) {
-        wx += coef * t.x;
-        wz += coef * t.z;
-    };
-    plane(-1.0 / 60.0, xz_cross_y(m2, c12));
-    const double y112 = xz_cross(m1, c112);
-    wy += (1.0 / 360.0) * y112;
-    plane(1.0 / 140.0, xz_cross_y(m2, c14));
-    plane(-1.0 / 420.0, xz_cross_y(m3, c13));
-    plane(-1.0 / 210.0, xz_cross_y(m4, c12));
-    wy += (-1.0 / 840.0) * xz_cross(m1, xz_cross_y(m1, c14));
-    wy += (1.0 / 504.0) * xz_cross(m2, c113);
-    wy += (-1.0 / 840.0) * xz_cross(m2, xz_cross_y(m2, c12));
-    wy += (1.0 / 2520.0) * xz_cross(m3, c112);
-    plane(-1.0 / 2520.0, xz_cross_y(m1, xz_cross(m1, c113)));
-    plane(-1.0 / 7560.0, y_cross_xz(c12, c112));
-    plane(1.0 / 2520.0, xz_cross_y(m2, y112));
-    wy += (-1.0 / 15120.0) * xz_cross(m1, xz_cross_y(m1, y112));
-    const double a = -wz, b = wy, c = -wx;
-    const double n2 = a * a + b * b + c * c;
-    const double ev = sqrt(n2);
-    double y, x;
-    sincos(ev, &y, &x);
-    const double in2 = 1.0 / n2;
-    const double s0 = S[0], s1 = S[1], s2 = S[2];
-    S[0] = (((a * a + b * b) * x + c * c) * s0 + (b * c * (x - 1) + a * ev * y) * s1 +
-            (-a * c * (x - 1) + b * ev * y) * s2) * in2;
-    S[1] = ((b * c * (x - 1) - a * ev * y) * s0 + ((a * a + c * c) * x + b * b) * s1 +
-            (a * b * (x - 1) + c * ev * y) * s2) * in2;
-    S[2] = ((-a * c * (x - 1) - b * ev * y) * s0 + (a * b * (x - 1) - c * ev * y) * s1 +
-            ((b * b + c * c) * x + a * a) * s2) * in2;
+// rotation_factors for angles up to 4 at a half or a quarter of the angle:
+// with a = sin(theta/2) / (theta/2), b = (1 - cos(theta/2)) / (theta/2)^2 and
+// cos(theta/2) = 1 - b x/4, sin(theta) / theta = a cos(theta/2) and
+// (1 - cos(theta)) / theta^2 = a^2 / 2.  The warp takes one path.
+__device__ __forceinline__ void rotation_double(double x4, double &sa, double &ca) {
+    const double a = sa;
+    sa = a * fma(-ca, x4, 1.0);
+    ca = 0.5 * (a * a);
+}
+__device__ __forceinline__ void rotation_factors_wide(double x, double &sa, double &ca) {
+    const unsigned m = __activemask();
+    if (__all_sync(m, x <= 4.0)) {
+        rotation_series(0.25 * x, sa, ca);
+        rotation_double(0.25 * x, sa, ca);
+    } else if (__all_sync(m, x <= 16.0)) {
+        rotation_series(0.0625 * x, sa, ca);
+        rotation_double(0.0625 * x, sa, ca);
+        rotation_double(0.25 * x, sa, ca);
+    } else {
+        const double2 f = rotation_factors_large(x);
+        sa = f.x;
+        ca = f.y;
+    }
 }
 
 // The error norm's denominator of component c after an attempt of size h:
@@ -2120,7 +2122,7 @@ bz_integrate_kernel(const KParams P) {
     constexpr bool kFree = Traits<M>::kRelax && PROPOSER == 0 && STEPPER == 0 && OUT == 0;
     // (Magnus-4: the header and the first substep's sums and differences)
     // (dyadic steppers: up to the end of the level-0 stage table)
-    constexpr int COPY = kFree           ? 2
+    constexpr int COPY = kFree || STEPPER == 2 ? 2
                          : STEPPER == 1  ? slot_poly(NF) + 2 * NF
                          : kDyadic       ? DYA + ((13 * NF + 1) & ~1)
                          : PROPOSER == 0 ? SLOT
@@ -2133,7 +2135,7 @@ bz_integrate_kernel(const KParams P) {
     constexpr bool kFetch = (STEPPER == 0 && (!kNarrow || kDyadic) && !kFree) || STEPPER == 1;
     __shared__ __align__(16) double stage_raw[kWarpsPerBlock][kFetch ? 2 : 1][COPY];
     __shared__ double free_ring[kWarpsPerBlock][kFree ? kFreeWindow * 32 : 1];
-    constexpr bool kRingSum = kFetch && OUT == 0;
+    constexpr bool kRingSum = (kFetch || STEPPER == 2) && OUT == 0;
     __shared__ double ring[kWarpsPerBlock][kRingSum ? kRing * kRingRow : 1];
     __shared__ __align__(16) V stage_tab[kWarpsPerBlock][kNarrow && PROPOSER == 0 ? NTAB : 1];
     // learned proposer: per-warp input tiles in dynamic shared memory
@@ -2201,14 +2203,6 @@ bz_integrate_kernel(const KParams P) {
             double held2 = 0.0; // ... and of its second channel (OUT 1)
             double kc[4];       // momentum cosines (OUT 1-3)
             if constexpr (OUT >= 1 && OUT <= 3) piflux_cosines(row, kc);
-            // closed-form Magnus step: the next interval's moments are loaded
-            // while the current step computes (registers, off the step's chain)
-            double mom_next[4] = {0.0, 0.0, 0.0, 0.0};
-            if constexpr (STEPPER == 2) {
-#pragma unroll
-                for (int c = 0; c < 4; ++c) mom_next[c] = __ldg(coef + TAB + c);
-            }
-
             if constexpr (CHUNK) {
                 for (int c = 0; c < chunk; ++c) apply_propagator(P, item, c, lane, S);
 #pragma unroll
@@ -2238,13 +2232,45 @@ bz_integrate_kernel(const KParams P) {
                             prow);
                 integrate_free<M, D>(P, pd, ms, coef, dt0, tb, te, N, w, dead, S, held, prow, sub, lane,
                                      free_ring[wib], my_attempts, my_rejects);
+            } else if constexpr (STEPPER == 2) {
+                // the interval's Legendre moments sit where the standard
+                // schedule's table would (staging layout 3) and are loaded one
+                // interval ahead; the model's vertex reads the state only
+                const DiracMagnus step(row[0], row[1], row[2], pd.measure_every);
+                const double *mo = coef + TAB;
+                double mom[4];
+                load_even<4>(mo, mom);
+                double *ko = OUT == 4 ? P.kout + q : nullptr;
+                for (int i = 0;; ++i) {
+                    const double c = dead ? 0.0 : w * ms.vertex(nullptr, S);
+                    if constexpr (OUT == 4) {
+                        if (valid) *ko = c;
+                        ko += P.n_k;
+                    } else {
+                        put_sample(i, c, N, sub, lane, ring[wib], prow);
+                    }
+                    if (i == N) break;
+                    double wv[3];
+                    step.omega(mom, wv);
+                    if (i + 1 < N) load_even<4>(mo += SLOT, mom);
+                    if (!dead) {
+                        double sa, ca;
+                        rotation_factors_wide(wv[0] * wv[0] + wv[1] * wv[1] + wv[2] * wv[2], sa, ca);
+                        rotate(wv, sa, ca, S);
+                        ++my_attempts;
+                        if (!(isfinite(S[0]) && isfinite(S[1]) && isfinite(S[2]))) {
+                            dead = true;
+                            atomicAdd(P.counters + 4, 1ull);
+                            atomicMax(P.status, 3);
+                        }
+                    }
+                }
             } else {
             for (int i = i0; i <= i_end; ++i) {
                 const double *rec = CHUNK && i0 > 0 ? coef + (size_t)(i0 - 1) * SLOT + 4 : pd.s0rec;
                 if (i > i0) {
-                    // interval i-1 in this warp's shared slot (the closed-form
-                    // Magnus step reads its moments and the record straight from
-                    // the staging table: warp broadcasts of a few values)
+                    // interval i-1 in this warp's shared slot (Magnus-4 with many
+                    // substeps reads the staging table: warp broadcasts)
                     const double *gslot = coef + (size_t)(i - 1) * SLOT;
                     if constexpr (kFetch) {
                         slot = stage_raw[wib][(i - 1) & 1];
@@ -2315,20 +2341,6 @@ bz_integrate_kernel(const KParams P) {
                                 rotate(wv, S);
                             }
                             my_attempts += ns;
-                        }
-                    } else if constexpr (STEPPER == 2) {
-                        // the interval's Legendre moments sit where the standard
-                        // schedule's table would (staging layout 3)
-                        double mom[4];
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) mom[c] = mom_next[c];
-                        if (i < N) {
-#pragma unroll
-                            for (int c = 0; c < 4; ++c) mom_next[c] = __ldg(gslot + SLOT + TAB + c);
-                        }
-                        if (!dead) {
-                            dirac_magnus_step(row[0], row[1], row[2], pd.measure_every, mom, S);
-                            ++my_attempts;
                         }
                     } else if constexpr (!kDyadic) {
                         const int n_std = (PROPOSER == 0) ? (int)slot[SCHED] : 0;
