@@ -1512,12 +1512,12 @@ struct DiracMagnus {
 };
 
 // rotation_factors for angles up to 4 at a half or a quarter of the angle:
-// with a = sin(theta/2) / (theta/2), b = (1 - cos(theta/2)) / (theta/2)^2 and
-// cos(theta/2) = 1 - b x/4, sin(theta) / theta = a cos(theta/2) and
-// (1 - cos(theta)) / theta^2 = a^2 / 2.  The warp takes one path.
-__device__ __forceinline__ void rotation_double(double x4, double &sa, double &ca) {
+// with a = sin(u) / u, b = (1 - cos(u)) / u^2 and cos(u) = 1 - b u^2, the
+// double angle has sin(2u) / 2u = a cos(u) and (1 - cos(2u)) / (2u)^2 = a^2 / 2.
+// The warp takes one path.
+__device__ __forceinline__ void rotation_double(double u2, double &sa, double &ca) {
     const double a = sa;
-    sa = a * fma(-ca, x4, 1.0);
+    sa = a * fma(-ca, u2, 1.0);
     ca = 0.5 * (a * a);
 }
 __device__ __forceinline__ void rotation_factors_wide(double x, double &sa, double &ca) {
@@ -2856,46 +2856,60 @@ static __global__ void kappa_rows_kernel(const KappaItem *__restrict__ items, in
 
 // One refinement level: item b updates its split's trapezoid estimate
 //   T[split][i] <- scale T + h sum_rows contrib[i][row]
-// (scale 0 on the first round, 1/2 after a halving) and writes change[b] =
-// max_i |T_new - T_old| (NaN if any sample is NaN).  One CTA per split, one
-// thread per sample: each thread adds the split's rows in order (its own
-// contiguous run, kept in L1 while it is read), a fixed order.
-constexpr int kKappaThreads = 256;
-__device__ __forceinline__ double nan_max(double a, double b) { return (b > a || b != b) ? b : a; }
+// (scale 0 on the first round, 1/2 after a halving) and raises change[b]
+// (zero before) to max_i |T_new - T_old| (NaN if any sample is NaN).  A CTA
+// takes kRoundItems consecutive items, whose rows follow each other, and 32
+// samples: the rows come in tiles through shared memory, each sample's with
+// coalesced loads, then thread (item, sample) adds its item's rows in order.
+// Read by the adding threads themselves, 80 bytes here and there, a warp's
+// loads touched 32 sectors each: 3.06 ms for 4.2 GB (63 800 rows x 8193 samples),
+// 1.40 ms now (3.0 TB/s).
+constexpr int kRoundItems = 8, kRoundSamples = 32, kRoundTile = 128;
+constexpr int kKappaThreads = kRoundItems * kRoundSamples;
 
 static __global__ void __launch_bounds__(kKappaThreads)
 kappa_round_kernel(const double *__restrict__ contrib, long long n_rows, int n_samples,
-                   const KappaItem *__restrict__ items, double *__restrict__ T,
-                   double *__restrict__ change) {
-    constexpr int kWarps = kKappaThreads / 32;
-    __shared__ double wmax[kWarps];
-    const KappaItem &it = items[blockIdx.x];
+                   const KappaItem *__restrict__ items, int n_items, double *__restrict__ T,
+                   unsigned long long *__restrict__ change) {
+    __shared__ double tile[kRoundSamples][kRoundTile + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double *Ts = T + (size_t)it.split * n_samples;
-    const double *c0 = contrib + it.row0;
-    const int n = it.n;
-    const double sc = it.level == 0 ? 0.0 : 0.5, hb = it.h;
-    double dmax = 0.0;
-    for (int i = threadIdx.x; i < n_samples; i += kKappaThreads) {
-        const double *c = c0 + (size_t)i * n_rows;
-        double acc = 0.0;
-#pragma unroll 4
-        for (int r = 0; r < n; ++r) acc += __ldg(c + r);
-        const double old = Ts[i];
+    const unsigned sample_blocks = ((unsigned)n_samples + kRoundSamples - 1) / kRoundSamples;
+    const int b0 = (int)(blockIdx.x / sample_blocks) * kRoundItems, b = b0 + warp;
+    const int s0 = (int)(blockIdx.x % sample_blocks) * kRoundSamples, i = s0 + lane;
+    const KappaItem &it = items[min(b, n_items - 1)];
+    const KappaItem &last = items[min(b0 + kRoundItems, n_items) - 1];
+    // items of one level follow each other in rows unless splits between them
+    // are done: each item's rows, the CTA's span
+    const long long lo = items[b0].row0, hi = last.row0 + last.n;
+    const long long r0 = it.row0, r1 = b < n_items ? it.row0 + it.n : it.row0;
+    double acc = 0.0;
+    for (long long t0 = lo; t0 < hi; t0 += kRoundTile) {
+        const int nt = (int)min((long long)kRoundTile, hi - t0);
+        // (also: the previous tile has been added) rows of finished splits are skipped
+        if (!__syncthreads_or(r0 < t0 + nt && r1 > t0)) continue;
+        for (int s = warp; s < kRoundSamples; s += kRoundItems) {
+            if (s0 + s >= n_samples) break;
+            const double *c = contrib + (size_t)(s0 + s) * n_rows + t0;
+            for (int r = lane; r < nt; r += 32) tile[s][r] = __ldcs(c + r);
+        }
+        __syncthreads();
+        const int a = (int)(max(r0, t0) - t0), e = (int)(min(r1, t0 + nt) - t0);
+        for (int r = a; r < e; ++r) acc += tile[lane][r];
+    }
+    double d = 0.0;
+    if (b < n_items && i < n_samples) {
+        double *Ts = T + (size_t)it.split * n_samples + i;
+        const double old = *Ts;
         // two rounded products and a rounded sum (no contraction)
-        const double v = __dadd_rn(__dmul_rn(sc, old), __dmul_rn(hb, acc));
-        Ts[i] = v;
-        dmax = nan_max(dmax, fabs(v - old));
+        const double v = __dadd_rn(__dmul_rn(it.level == 0 ? 0.0 : 0.5, old), __dmul_rn(it.h, acc));
+        *Ts = v;
+        d = fabs(v - old);
     }
+    // non-negative doubles compare as their bit patterns, NaN above all
+    unsigned long long m = (unsigned long long)__double_as_longlong(d);
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) dmax = nan_max(dmax, __shfl_xor_sync(kFull, dmax, o));
-    if (lane == 0) wmax[warp] = dmax;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double m = 0.0;
-        for (int w = 0; w < kWarps; ++w) m = nan_max(m, wmax[w]);
-        change[blockIdx.x] = m;
-    }
+    for (int o = 16; o >= 1; o >>= 1) m = max(m, __shfl_xor_sync(kFull, m, o));
+    if (lane == 0 && b < n_items) atomicMax(change + b, m);
 }
 
 // j[i] = dz * sum over slices (in order) of the slice's sum over its splits

@@ -2658,8 +2658,13 @@ hhg_status dirac_quadrature(hhg_ctx *ctx, const hhg_system_desc *sys, const hhg_
                 const int nt = (int)todo.size();
                 HHG_CUDA(ctx, cudaMemcpyAsync(ditems, todo.data(), nt * sizeof(hhg::KappaItem),
                                               cudaMemcpyHostToDevice, s));
-                hhg::kappa_round_kernel<<<nt, hhg::kKappaThreads, 0, s>>>(
-                    pl->d_kout, std::max(n_rows, 1LL), n_samples, ditems, dT, dchange);
+                HHG_CUDA(ctx, cudaMemsetAsync(dchange, 0, nt * sizeof(double), s));
+                const unsigned round_grid =
+                    (unsigned)((nt + hhg::kRoundItems - 1) / hhg::kRoundItems) *
+                    (unsigned)((n_samples + hhg::kRoundSamples - 1) / hhg::kRoundSamples);
+                hhg::kappa_round_kernel<<<round_grid, hhg::kKappaThreads, 0, s>>>(
+                    pl->d_kout, std::max(n_rows, 1LL), n_samples, ditems, nt, dT,
+                    reinterpret_cast<unsigned long long *>(dchange));
                 HHG_CUDA(ctx, cudaGetLastError());
                 // the context stream does not synchronise with the legacy
                 // stream: copies are ordered on it
