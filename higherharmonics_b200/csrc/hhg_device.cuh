@@ -17,18 +17,19 @@
 //    schedule": the reference restarts every interval at dt0 = measure_every /
 //    n_subdivisions (PiFlux.cpp:98,105), and a trajectory whose error stays
 //    below 5^-8 grows dt by exactly 0.9 * 5 each step, so every such lane takes
-//    the same (t, dt) sequence.  When all active lanes of a warp are on that
-//    schedule (a warp vote per attempt) the right-hand sides read the
-//    tabulated values with broadcast shared-memory loads.
+//    the same (t, dt) sequence.  While all lanes of a warp are on that
+//    schedule the warp takes its steps (one vote an attempt) and the
+//    right-hand sides read the tabulated values with broadcast shared-memory
+//    loads.
 // In the mixed-precision variant the right-hand sides and the stage sums are
 // FP32 (products of the FP32-rounded pulse values and k-dependent constants);
 // the state, the solution and error increments, the error norm and the step
 // control are FP64.
 //
-// At every sample the lanes' weighted current contributions are reduced with a
-// butterfly shuffle; lane (i mod 32) keeps sample i and every 32 samples the
-// warp stores its 32 sums with one coalesced 256-byte store into the work
-// item's row of the partial buffer.  Work items are taken from a global atomic
+// The lanes' weighted current contributions of eight samples at a time are
+// summed through shared memory (put_sample; the variants without it: a
+// butterfly shuffle per sample, kept by lane (i mod 32)) and stored into the
+// work item's row of the partial buffer.  Work items are taken from a global atomic
 // counter (persistent, work-stealing launch), and a second kernel reduces the
 // partial rows of each pulse in item order with compensated sums, so j(t) is
 // bitwise reproducible whatever the schedule.
@@ -49,8 +50,9 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr double kDblEps = 2.220446049250313080847e-16;  // std::numeric_limits<double>::epsilon()
 constexpr double kErrScale = 840.0 / 41.0;  // 1 / the error estimate's 41/840 (error_den)
 constexpr int kMaxStd = 5;  // tabulated steps of the standard schedule per interval
-// Integration CTAs are 2 warps; at <= 144 registers 7 CTAs (14 warps) fit an
-// SM, so a 256x256 grid (2048 warps) is resident in a single wave on 148 SMs.
+// Integration CTAs are 2 warps (1 or 4 measured the same).  7 CTAs per SM are
+// 128 registers a thread (14 warps, up to 4 per scheduler); variants that do
+// better with fewer warps and more registers: min_blocks().
 constexpr int kWarpsPerBlock = 2;
 constexpr int kBlockThreads = 32 * kWarpsPerBlock;
 constexpr int kMinBlocksPerSM = 7;
@@ -2147,7 +2149,10 @@ bz_integrate_kernel(const KParams P) {
     const int wib = threadIdx.x >> 5;
     double *slot = stage_raw[wib][0];
 
-    static_assert(!CHUNK || (!kNarrow && kFetch && PROPOSER == 0 && OUT != 1), "chunked variants");
+    // variants with a chunked form (chunk_variant)
+    constexpr bool kChunkable = !kNarrow && kFetch && PROPOSER == 0 && OUT != 1 && OUT != 4 && D != 0 &&
+                                !Traits<M>::kRelax;
+    static_assert(!CHUNK || kChunkable, "chunked variants");
     __shared__ double chunk_s0[kWarpsPerBlock][CHUNK ? 96 : 1];  // the chunk's start state
 
     unsigned long long my_attempts = 0, my_rejects = 0;
@@ -2162,9 +2167,11 @@ bz_integrate_kernel(const KParams P) {
             item /= P.n_chunks;
         }
         const int p = (int)(item / P.items_per_pulse);
-        if (CHUNK || P.only_discarded) {
-            const bool off = chunk_discarded(P, p, lane);
-            if (CHUNK ? off : !off) continue;
+        if constexpr (kChunkable) {
+            if (CHUNK || P.only_discarded) {
+                const bool off = chunk_discarded(P, p, lane);
+                if (CHUNK ? off : !off) continue;
+            }
         }
         const int tile = (int)(item % P.items_per_pulse);
         const PulseDev &pd = P.pulses[p];
