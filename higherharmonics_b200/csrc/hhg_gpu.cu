@@ -1102,10 +1102,11 @@ hhg_status hhg_grid_rows(const hhg_system_desc *sys, const hhg_grid_desc *grid, 
 
 // cost_order: for the PiFlux-3D models, order the k rows by a cost
 // proxy (below); plans whose outputs are indexed by k keep the caller's order.
+// out_mode: bz_integrate_kernel's OUT.
 static hhg_status plan_create_impl(hhg_ctx *ctx, const hhg_system_desc *sys,
                                    const hhg_pulse_desc *pulses, int n_pulses,
                                    const hhg_grid_desc *grid, const hhg_solver_opts *opts,
-                                   hhg_plan **out, bool cost_order) {
+                                   hhg_plan **out, bool cost_order, int out_mode = 0) {
     if (!ctx || !out) return HHG_BAD_CONFIG;
     *out = nullptr;
     hhg_status st = check_system(ctx, sys);
@@ -1158,6 +1159,7 @@ static hhg_status plan_create_impl(hhg_ctx *ctx, const hhg_system_desc *sys,
     pl->ctx = ctx;
     pl->model = kernel_model(*sys);
     pl->opts = o;
+    pl->out_mode = out_mode;
     pl->n_pulses = n_pulses;
     const int nf = model_nf(pl->model);
 
@@ -2264,7 +2266,7 @@ hhg_status output_plan(hhg_ctx *ctx, const hhg_system_desc *sys, const hhg_pulse
                            "k-resolved and split-current outputs run FP64 RKF78 with the NONE or CARRY proposer");
     }
     hhg_plan *pl = nullptr;
-    hhg_status st = plan_create_impl(ctx, sys, pulse, 1, grid, &o, &pl, false);  // k order kept
+    hhg_status st = plan_create_impl(ctx, sys, pulse, 1, grid, &o, &pl, false, mode);  // k order kept
     if (st != HHG_OK) return st;
     if (pl->degree == 0) {
         hhg_plan_destroy(pl);
@@ -2277,8 +2279,6 @@ hhg_status output_plan(hhg_ctx *ctx, const hhg_system_desc *sys, const hhg_pulse
         return set_err(ctx, HHG_CUDA_ERROR, std::string(what) + ": " + cudaGetErrorString(e));
     };
     cudaError_t e;
-    pl->out_mode = mode;
-    setup_chunks(pl);
     if (mode == 1) {  // a second channel of partial rows and of j
         cudaFree(pl->d_part);
         cudaFree(pl->d_j);
@@ -2465,15 +2465,14 @@ hhg_status dirac_quadrature(hhg_ctx *ctx, const hhg_system_desc *sys, const hhg_
         ctx->kappa_key.clear();
         ctx->kappa_cap = 0;
         hhg_plan *np = nullptr;
-        if ((st = hhg_plan_create(ctx, sys, pulse, 1, &g, &o, &np)) != HHG_OK) return st;
+        // (no intervals in parallel: the launches vary in size)
+        if ((st = plan_create_impl(ctx, sys, pulse, 1, &g, &o, &np, true, 4)) != HHG_OK) return st;
         if (np->degree == 0) {
             hhg_plan_destroy(np);
             return set_err(ctx, HHG_UNSUPPORTED,
                            "spline pulse too steep for the staged interpolants: its exact "
                            "evaluation runs the Brillouin-zone current only");
         }
-        np->out_mode = 4;
-        setup_chunks(np);  // none: the launches vary in size
         int occ = 0;
         hhg::LaunchReq lr{};
         lr.degree = np->degree;
