@@ -944,12 +944,20 @@ hhg_status check_relax(hhg_ctx *ctx, const hhg_system_desc &s, const hhg_pulse_d
 // Intervals in parallel for plans of at most one 32-row tile per SM.  The
 // chunked run does about 3.5 times the arithmetic of the sequential one (the
 // three basis vectors, then the run); one warp alone keeps its scheduler's
-// FP64 pipe 40-80 % busy, so T tiles break even near T = 256 of the 592
-// schedulers (gapped Dirac, 4096 intervals: T = 32 9.0 -> 1.3 ms, T = 145 9.0
-// -> 5.9 ms).  A pulse's chunks, for about 12 warps per SM (4 lose 10-25 %) and
-// a multiple of the sample block, follow from its own tiles and intervals
-// alone, so pulses agree bit for bit with their single runs in every plan that
-// runs in chunks.
+// FP64 pipe 40-80 % busy, so the two break even near 225 tiles (4096 intervals,
+// sequential / chunked ms: gapped Dirac 32 tiles 8.9 / 1.4, 128 9.0 / 5.5, 145
+// 9.0 / 5.9, 162 9.0 / 7.1, 221 9.0 / 8.7, 254 9.0 / 11.8; honeycomb 10.7 / 6.7
+// at 145, 10.7 / 10.0 at 221).  The line lies at one tile per SM because a pulse
+// that leaves the schedule pays for both: about 1 % where the propagators meet
+// it, and the whole chunked run where only the chunks' ends show it (honeycomb,
+// 128 tiles, energy scale 28: 8.6 ms, sequential 5.4; its neighbours 25 and 30
+// do not).  Beyond 148 tiles that price is 1.8 and more for a gain below 1.3.
+// The plan's first execution pays it; the discard is a property of the plan's
+// inputs and is kept with them (enqueue_integration).
+// A pulse's chunks, for about 12 warps per SM (4 lose 10-25 %) and a multiple
+// of the sample block, follow from its own tiles and intervals alone, so pulses
+// agree bit for bit with their single runs in every plan that runs in chunks
+// (with a plan that does not: up to rounding).
 constexpr int kChunkWarpsPerSm = 12, kMaxChunks = 128, kMinChunks = 4;
 void setup_chunks(hhg_plan *pl) {
     pl->n_chunks = 1;
@@ -970,10 +978,14 @@ void setup_chunks(hhg_plan *pl) {
         !hhg::chunk_variant(pl->model, pl->degree, pl->opts.precision, pl->opts.stepper,
                             kernel_proposer(pl->opts.proposer), pl->opts.magnus_substeps, pl->out_mode))
         return;
-    if (cudaMalloc(&pl->d_chunk_stat, sizeof(unsigned long long) * hhg::kChunkStat * pl->n_pulses) != cudaSuccess ||
-        cudaMalloc(&pl->d_prop, sizeof(double) * 9 * 32 * (size_t)pl->n_items * most) != cudaSuccess) {
+    const size_t stat_bytes = sizeof(unsigned long long) * hhg::kChunkStat * pl->n_pulses;
+    if (cudaMalloc(&pl->d_chunk_stat, stat_bytes) != cudaSuccess ||
+        cudaMalloc(&pl->d_prop, sizeof(double) * 9 * 32 * (size_t)pl->n_items * most) != cudaSuccess ||
+        cudaMemsetAsync(pl->d_chunk_stat, 0, stat_bytes, ctx->stream) != cudaSuccess ||
+        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
         cudaGetLastError();  // no room: the sequential run needs none
         cudaFree(pl->d_chunk_stat);
+        cudaFree(pl->d_prop);
         pl->d_chunk_stat = nullptr;
         pl->d_prop = nullptr;
         return;
@@ -1576,9 +1588,12 @@ hhg_status enqueue_integration(hhg_plan *pl, cudaStream_t s, bool events) {
     hhg_status st = HHG_OK;
     if (pl->n_chunks > 1) {
         // the chunks' propagators, the chunked run, and the sequential run of the
-        // pulses whose chunked one was discarded
-        HHG_CUDA(ctx, cudaMemsetAsync(pl->d_chunk_stat, 0,
-                                      sizeof(unsigned long long) * hhg::kChunkStat * pl->n_pulses, s));
+        // pulses whose chunked one was discarded.  That follows from the plan's
+        // pulse, rows and tolerances, so the flag (word 0) is set once: later
+        // executions of the plan run the pulse sequentially at once, with the
+        // same bits.  The step counts start at zero each time.
+        HHG_CUDA(ctx, cudaMemset2DAsync(pl->d_chunk_stat + 1, sizeof(unsigned long long) * hhg::kChunkStat, 0,
+                                        sizeof(unsigned long long) * (hhg::kChunkStat - 1), pl->n_pulses, s));
         hhg::LaunchReq cr = lr;
         cr.kp.prop = pl->d_prop;
         cr.kp.n_chunks = pl->n_chunks;
