@@ -376,9 +376,7 @@ template <typename R> struct Num;
 template <> struct Num<double> {
     using V = double;  // pulse value / k constant
     static __device__ __forceinline__ V mk(double x) { return x; }
-    static __device__ __forceinline__ double lin(V a, V b, V f) { return a - b * f; }       // a - b f
     static __device__ __forceinline__ double dot2(V a, V b, V c, V d) { return a * b + c * d; }
-    static __device__ __forceinline__ double mul(V a, V f) { return a * f; }
 };
 template <> struct Num<float> {
     using V = float2;
@@ -387,7 +385,7 @@ template <> struct Num<float> {
         return make_float2(h, (float)(x - (double)h));
     }
     // compensated products: each field term gets one final FP32 rounding
-    static __device__ __forceinline__ float lin(V a, V b, V f) {
+    static __device__ __forceinline__ float lin(V a, V b, V f) {  // a - b f
         const float lo = a.y - b.x * f.y - b.y * f.x;
         return fmaf(-b.x, f.x, a.x) + lo;
     }
@@ -746,16 +744,13 @@ template <typename R, bool X> struct HoneycombState {
         py = p.mp[3];
     }
     // pf Re gamma', pf Im gamma' with e^{i(a - b)} = (ca cb + sa sb) + i (sa cb - ca sb)
+    // (the X models form theirs in node() and node32())
     __device__ __forceinline__ void gamma(const typename N::V *f, R &gr, R &gi) const {
-        if constexpr (X) {
-            gr = R(N::dot2(pc0, f[0], ps0, f[1])) + R(N::dot2(pc1, f[2], ps1, f[3]));
-            gi = R(N::dot2(ps0, f[0], mc0, f[1])) + R(N::dot2(ps1, f[2], mc1, f[3]));
-        } else {
-            gr = R(N::dot2(pc0, f[0], ps0, f[1])) + R(N::dot2(pc1, f[2], ps1, f[3])) +
-                 R(N::dot2(pc2, f[Q2], ps2, f[Q2 + 1]));
-            gi = R(N::dot2(ps0, f[0], mc0, f[1])) + R(N::dot2(ps1, f[2], mc1, f[3])) +
-                 R(N::dot2(ps2, f[Q2], mc2, f[Q2 + 1]));
-        }
+        static_assert(!X, "three bonds");
+        gr = R(N::dot2(pc0, f[0], ps0, f[1])) + R(N::dot2(pc1, f[2], ps1, f[3])) +
+             R(N::dot2(pc2, f[Q2], ps2, f[Q2 + 1]));
+        gi = R(N::dot2(ps0, f[0], mc0, f[1])) + R(N::dot2(ps1, f[2], mc1, f[3])) +
+             R(N::dot2(ps2, f[Q2], mc2, f[Q2 + 1]));
     }
     // FP64: the bond sums from the momentum cosines kept for the vertex
     struct Step {
@@ -1606,11 +1601,11 @@ __device__ __forceinline__ bool control(const KParams &P, const double *S, const
 // whole warp: pulse values from the table, no per-lane t and dt, and one vote
 // an attempt.  The first attempt that takes a lane off the schedule is
 // finished by the per-lane controller, which then goes on with the
-// interpolants.  Before, every lane ran its own controller on the table path
-// too: votes on t and dt, and at the ends of the third and fourth step of an
-// interval three quotients and a power.  With the records one interval ahead
-// and the samples summed in blocks: pi-flux 256 x 256 (8192 intervals) 76.6 ->
-// 54.6 ms, gapped Dirac 64 x 64 14.0 -> 9.3 ms.
+// interpolants.  A controller per lane on the table path costs votes on t and
+// dt, and at the ends of the third and fourth step of an interval three
+// quotients and a power: pi-flux 256 x 256 (8192 intervals) 76.6 ms that way,
+// 54.6 this way, with the records one interval ahead and the samples summed in
+// blocks.
 // ---------------------------------------------------------------------------
 template <int M, int NF, int D, typename R, bool USE_STD, bool CARRY, bool REC = false>
 __device__ __forceinline__ void lane_controller(const KParams &P, const ModelState<M, R> &ms,
@@ -1738,34 +1733,6 @@ __device__ __forceinline__ void copy16_async(void *smem, const void *gmem) {
                  : "memory");
 }
 
-// ---------------------------------------------------------------------------
-// Persistent, work-stealing integration + BZ-sum kernel.
-// STEPPER 0: controlled RKF78; STEPPER 1: Magnus-4 (two-point Gauss),
-//   magnus_substeps steps per interval: omega = h (d1 + d2) + (sqrt3/3) h^2
-//   (d2 x d1), S <- exp([omega]_x) S, from the staged sums and differences
-//   (up to kMagnusTab substeps; STEPPER 3: more, from the interpolants).  The
-//   Gauss-point values, formerly two interpolants per staged function
-//   evaluated by every lane, and the rotation (a root, a sine and cosine, two
-//   quotients) were two thirds of the 199 FP64 instructions of an interval
-//   (honeycomb):
-//   512 x 512, 6144 intervals, 42.7 -> 15.2 ms a spectrum, 89 FP64 instructions.
-// PROPOSER 0: the reference's per-lane controller, every interval restarting
-//   at dt0 = measure_every / n_subdivisions;
-// PROPOSER 1: per-lane controller, an interval starts from the controller's
-//   last proposal of the previous interval;
-// PROPOSER 2: warp-synchronous dyadic stepping: all lanes of a warp take the
-//   step (t1 - t0) / 2^L at positions q of the dyadic grid; the step is
-//   accepted only if every lane's embedded error passes (|e_i| <= abs + rel
-//   (|x_i| + h |dxdt_i|), the reference's norm), otherwise the warp retries at
-//   L + 1; after an accepted step the warp coarsens when every lane's error
-//   would still pass at twice the step (err < 1/600 ~ 0.9^8 / 2^8) and q is
-//   even.  Levels below kDyaLevels read the tabulated pulse values from the
-//   staging slot (global memory, broadcast within the warp); beyond
-//   kLevelMax the warp falls back to the per-lane controller.  The level is
-//   carried to the next interval.
-// The mixed-precision variant (R = float) evaluates the growth/shrink factor's
-// power in FP32 (the error norm, the comparison and dt stay FP64).
-// ---------------------------------------------------------------------------
 // ---------------------------------------------------------------------------
 // Free-running lanes (the relaxation models on the reference schedule, BZ
 // sum): every lane integrates its own intervals with the per-lane controller
@@ -2075,25 +2042,17 @@ constexpr int kCoarsenDivMixed = 64;
 // worth more than a fourth warp: 7 -> 5 CTAs, honeycomb 512 x 512 8.08 ->
 // 7.35 ms (256 intervals), pi-flux 256 x 256 3.47 -> 3.37 ms (512 intervals).
 // The lattice models' relaxation: 4 (255 registers; at 168 the stage values
-// spill, 1.7x slower).  Mixed precision: 7 (128 registers), pi-flux 5 (1.62 ->
-// 1.54 ms at 256 x 256 and 1024 intervals; honeycomb and Dirac lose 1-9 %).
+// spill, 1.7x slower).  Mixed precision: 7 (128 registers), except pi-flux,
+// whose compensated products of two projections spill there (lockstep, degree
+// 7: 142 bytes; 8 at 168 registers, 5 CTAs; 1.62 -> 1.54 ms at 256 x 256 and
+// 1024 intervals).  Dirac does not spill at 128, honeycomb with the field along
+// x by 24 bytes: they lose 1-9 % with 5.
 __host__ __device__ constexpr int min_blocks(int model, bool fp64, int stepper) {
     return model == PIFLUX3D_RELAX || model == HONEYCOMB_RELAX ? 4
            : fp64 ? (stepper == 0 ? 5 : kMinBlocksPerSM)
            : model == PIFLUX2D || model == PIFLUX2D_SYM ? 5 : kMinBlocksPerSM;
 }
 
-// OUT 0: the Brillouin-zone sum of the current (one partial row per item);
-// OUT 1: the same split by the instantaneous energy |d(k - A(t_i))| < energy_cut
-//   into two channels (PiFlux::current_per_energy, PiFlux.cpp:955-1035);
-// OUT 2: every trajectory's Bloch vector at every sample, kout[i][k][3];
-// OUT 3: every trajectory's band occupations at every sample, kout[i][k][2]
-//   (PiFlux::evolve_occupation_numbers, PiFlux.cpp:222-318);
-// OUT 4: every trajectory's weighted current w_k vertex(S) at every sample,
-//   kout[i][k], sample-major (a warp's store is one 256-byte run) (the kappa
-//   integrand of DiracSystem::compute_current_density,
-//   DiracSystem.cpp:300-311; dead trajectories give 0 and are counted).
-// OUT 1-3 are built for the PiFlux models only, OUT 4 for the Dirac-3D ones.
 // A warp's attempted and rejected steps into counters [1] and [2].
 __device__ __forceinline__ void add_steps(unsigned long long *counters, unsigned long long attempts,
                                           unsigned long long rejects, int lane) {
@@ -2108,8 +2067,48 @@ __device__ __forceinline__ void add_steps(unsigned long long *counters, unsigned
     }
 }
 
+// ---------------------------------------------------------------------------
+// Persistent, work-stealing integration + BZ-sum kernel.
+// STEPPER 0: controlled RKF78; STEPPER 1: Magnus-4 (two-point Gauss),
+//   magnus_substeps steps per interval: omega = h (d1 + d2) + (sqrt3/3) h^2
+//   (d2 x d1), S <- exp([omega]_x) S, from the staged sums and differences
+//   (up to kMagnusTab substeps; STEPPER 3: more, from the interpolants).  The
+//   two interpolants per staged function that every lane would evaluate for
+//   its Gauss points, and a rotation by its closed form (a root, a sine and
+//   cosine, two quotients), are 110 of 199 FP64 instructions of an interval:
+//   honeycomb 512 x 512, 6144 intervals, 42.7 ms a spectrum with them, 15.2
+//   without; STEPPER 2: the Dirac-3D closed-form step (DiracMagnus).
+// PROPOSER 0: the reference's per-lane controller, every interval restarting
+//   at dt0 = measure_every / n_subdivisions;
+// PROPOSER 1: per-lane controller, an interval starts from the controller's
+//   last proposal of the previous interval (PROPOSER 4: with step histories);
+// PROPOSER 2: warp-synchronous dyadic stepping: all lanes of a warp take the
+//   step (t1 - t0) / 2^L at positions q of the dyadic grid; the step is
+//   accepted only if every lane's embedded error passes (|e_i| <= abs + rel
+//   (|x_i| + h |dxdt_i|), the reference's norm), otherwise the warp retries at
+//   L + 1; after an accepted step the warp coarsens when every lane's error
+//   would still pass at twice the step (err < 1/600 ~ 0.9^8 / 2^8) and q is
+//   even.  Levels below kDyaLevels read tabulated pulse values, level 0 from
+//   the record in shared memory, the others from the staging slot (global
+//   memory, broadcast within the warp); beyond kLevelMax the warp falls back to
+//   the per-lane controller.  The level is carried to the next interval;
+// PROPOSER 3: the same with levels proposed by the network.
+// The mixed-precision variant (R = float) evaluates the growth/shrink factor's
+// power in FP32 (the error norm, the comparison and dt stay FP64).
+// OUT 0: the Brillouin-zone sum of the current (one partial row per item);
+// OUT 1: the same split by the instantaneous energy |d(k - A(t_i))| < energy_cut
+//   into two channels (PiFlux::current_per_energy, PiFlux.cpp:955-1035);
+// OUT 2: every trajectory's Bloch vector at every sample, kout[i][k][3];
+// OUT 3: every trajectory's band occupations at every sample, kout[i][k][2]
+//   (PiFlux::evolve_occupation_numbers, PiFlux.cpp:222-318);
+// OUT 4: every trajectory's weighted current w_k vertex(S) at every sample,
+//   kout[i][k], sample-major (a warp's store is one 256-byte run) (the kappa
+//   integrand of DiracSystem::compute_current_density,
+//   DiracSystem.cpp:300-311; dead trajectories give 0 and are counted).
+// OUT 1-3 are built for the PiFlux models only, OUT 4 for the Dirac-3D ones.
 // CHUNK: an item is one chunk of a tile's intervals, started from the state
 // that the propagators of the chunks before it give (chunk_propagator_kernel).
+// ---------------------------------------------------------------------------
 template <int M, int D, typename R, int STEPPER, int PROPOSER, int OUT = 0, bool CHUNK = false>
 __global__ void __launch_bounds__(kBlockThreads, min_blocks(M, sizeof(R) == sizeof(double), STEPPER))
 bz_integrate_kernel(const KParams P) {
@@ -2124,12 +2123,12 @@ bz_integrate_kernel(const KParams P) {
     constexpr int DYA = slot_dyadic(NF, D);
     constexpr bool kNarrow = sizeof(R) != sizeof(double);
     constexpr int kPair = pair_layout<M, R>();
-    // only the reference schedule reads the standard table; the dyadic table
-    // is read from global memory
     // the relaxation models on the reference schedule run free lanes (above)
     constexpr bool kFree = Traits<M>::kRelax && PROPOSER == 0 && STEPPER == 0 && OUT == 0;
-    // (Magnus-4: the header and the first substep's sums and differences)
-    // (dyadic steppers: up to the end of the level-0 stage table)
+    // The part of an interval's record in shared memory: the reference schedule
+    // all of it, Magnus-4 the header and the first substep's sums and
+    // differences, dyadic steppers up to the end of the level-0 stage table
+    // (the other levels are read from global memory), else up to the schedule.
     constexpr int COPY = kFree || STEPPER == 2 ? 2
                          : STEPPER == 1  ? slot_poly(NF) + 2 * NF
                          : kDyadic       ? DYA + ((13 * NF + 1) & ~1)
@@ -2137,9 +2136,9 @@ bz_integrate_kernel(const KParams P) {
                                          : SCHED;
     constexpr int NTAB = kMaxStd * 13 * NF;
     using V = typename Num<R>::V;
-    // FP64 RKF78 and Magnus-4: interval records are copied one interval ahead
-    // (cp.async) into two buffers, and samples are summed eight at a time
-    // (put_sample)
+    // FP64 RKF78, the dyadic steppers of both precisions and Magnus-4: interval
+    // records are copied one interval ahead (cp.async) into two buffers, and
+    // samples are summed eight at a time (put_sample)
     constexpr bool kFetch = (STEPPER == 0 && (!kNarrow || kDyadic) && !kFree) || STEPPER == 1;
     __shared__ __align__(16) double stage_raw[kWarpsPerBlock][kFetch ? 2 : 1][COPY];
     __shared__ double free_ring[kWarpsPerBlock][kFree ? kFreeWindow * 32 : 1];
