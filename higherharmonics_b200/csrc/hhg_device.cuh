@@ -2047,14 +2047,19 @@ constexpr int kCoarsenDivMixed = 64;
 // worth more than a fourth warp: 7 -> 5 CTAs, honeycomb 512 x 512 8.08 ->
 // 7.35 ms (256 intervals), pi-flux 256 x 256 3.47 -> 3.37 ms (512 intervals).
 // The lattice models' relaxation: 4 (255 registers; at 168 the stage values
-// spill, 1.7x slower).  Mixed precision: 7 (128 registers), except pi-flux,
-// whose compensated products of two projections spill there (lockstep, degree
-// 7: 142 bytes; 8 at 168 registers, 5 CTAs; 1.62 -> 1.54 ms at 256 x 256 and
-// 1024 intervals).  Dirac does not spill at 128, honeycomb with the field along
-// x by 24 bytes: they lose 1-9 % with 5.
-__host__ __device__ constexpr int min_blocks(int model, bool fp64, int stepper) {
+// spill, 1.7x slower).  Mixed precision: 7 (128 registers), except where the
+// compensated products of several projections spill there (lockstep, bytes at
+// 128 / 168 / 255 registers).  Pi-flux, degree 7, 142 / 8: 5 (1.62 -> 1.54 ms at
+// 256 x 256 and 1024 intervals).  Honeycomb off the axes, degree 7, 1258 / 160
+// / 8: 5 (256 intervals at 1024 per cycle, ms with 7 / 5 / 4: 200 x 200 0.54 /
+// 0.53 / 0.59, 512 x 512 2.30 / 2.33 / 2.45); degree 11, 3530 / 1794 / 40: 4 (64
+// per cycle and twice the field: 14.7 / 9.8 / 7.0 and 43.6 / 30.4 / 26.5).
+// Dirac does not spill at 128, honeycomb with the field along x by 24 bytes:
+// they lose 1-9 % with 5.
+__host__ __device__ constexpr int min_blocks(int model, bool fp64, int stepper, int degree) {
     return model == PIFLUX3D_RELAX || model == HONEYCOMB_RELAX ? 4
            : fp64 ? (stepper == 0 ? 5 : kMinBlocksPerSM)
+           : model == HONEYCOMB ? (degree == 11 ? 4 : 5)
            : model == PIFLUX2D || model == PIFLUX2D_SYM ? 5 : kMinBlocksPerSM;
 }
 
@@ -2115,7 +2120,7 @@ __device__ __forceinline__ void add_steps(unsigned long long *counters, unsigned
 // that the propagators of the chunks before it give (chunk_propagator_kernel).
 // ---------------------------------------------------------------------------
 template <int M, int D, typename R, int STEPPER, int PROPOSER, int OUT = 0, bool CHUNK = false>
-__global__ void __launch_bounds__(kBlockThreads, min_blocks(M, sizeof(R) == sizeof(double), STEPPER))
+__global__ void __launch_bounds__(kBlockThreads, min_blocks(M, sizeof(R) == sizeof(double), STEPPER, D))
 bz_integrate_kernel(const KParams P) {
     constexpr int NF = Traits<M>::NF;
     constexpr bool kDyadic = PROPOSER == 2 || PROPOSER == 3;
